@@ -1,0 +1,80 @@
+"""The tensor-core attention over the forms it takes: head sizes, query heads per kv head, lengths around its 16-position
+chunks, its 64-position slices and its splits.  Each call is compared with the float64 statement and with the general
+kernel on the same values (a cache that starts 4 bytes off a 16-byte boundary takes that one).
+
+Tolerance: a bf16 output (8 significant bits) is within half a unit in the last place, 2^-8 of the value; the 32-bit sums in
+between within 2^-16 of the largest weighted value (a few hundred roundings of 2^-24)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def both(n_head, n_kv, hd, lengths, seed=0, edit=None):
+    import torch
+    from turbo_lossless_b200 import Split12Engine
+    eng = Split12Engine()
+    rng = np.random.default_rng(seed)
+    B, T = len(lengths), max(lengths)
+    c = dict(q=rng.standard_normal((B, n_head * hd)).astype(np.float32),
+             k=rng.integers(-127, 128, (B, T, n_kv, hd)).astype(np.int8), v=rng.integers(-127, 128, (B, T, n_kv, hd)).astype(np.int8),
+             sk=(rng.random((B, T, n_kv)) * 0.03).astype(np.float32), sv=(rng.random((B, T, n_kv)) * 0.03).astype(np.float32))
+    c["k"][..., 0] = -128; c["v"][..., 1] = -128                       # the whole int8 range counts
+    if edit:
+        edit(c)
+    pos = torch.from_numpy(np.array(lengths, np.int32) - 1).cuda()
+    d = {n: torch.from_numpy(a).cuda() for n, a in c.items()}
+    outs = []
+    for off in (0, 4):
+        kv = []
+        for n in ("k", "v"):
+            room = torch.zeros(d[n].numel() + 16, dtype=torch.int8, device="cuda")
+            assert room.data_ptr() % 16 == 0
+            room[off:off + d[n].numel()] = d[n].flatten()
+            kv.append(room[off:])
+        out = torch.zeros(B, n_head * hd, dtype=torch.int16, device="cuda")
+        eng.attention_all_heads_batch(d["q"], kv[0], kv[1], d["sk"], d["sv"], out, pos, n_head, n_kv, hd, T,
+                                      1.0 / float(np.sqrt(hd)), B, T * n_kv * hd)
+        outs.append(out.view(torch.bfloat16).double().cpu().numpy())
+    return c, outs
+
+
+def exact(c, b, n, n_head, n_kv, hd):
+    g = n_head // n_kv
+    k = c["k"][b, :n].astype(np.float64) * c["sk"][b, :n].astype(np.float64)[..., None]
+    v = c["v"][b, :n].astype(np.float64) * c["sv"][b, :n].astype(np.float64)[..., None]
+    s = np.einsum("hgd,thd->hgt", c["q"][b].astype(np.float64).reshape(n_kv, g, hd), k) / np.sqrt(hd)
+    p = np.exp(s - s.max(axis=-1, keepdims=True))
+    p /= p.sum(axis=-1, keepdims=True)
+    return np.einsum("hgt,thd->hgd", p, v).reshape(-1), np.einsum("hgt,thd->hgd", p, np.abs(v)).reshape(-1)
+
+
+@pytest.mark.parametrize("hd", [64, 96, 128])
+@pytest.mark.parametrize("n_head,n_kv", [(1, 1), (4, 2), (8, 2), (16, 2), (32, 8)])
+@pytest.mark.parametrize("lengths", [(1,), (15, 16, 17), (63, 64, 65, 1), (127, 130, 2, 33), (1000, 520), (9,) * 40])
+def test_against_float64_and_the_general_kernel(hd, n_head, n_kv, lengths):
+    c, (new, general) = both(n_head, n_kv, hd, lengths, seed=hd + n_head + len(lengths))
+    for b, n in enumerate(lengths):
+        want, size = exact(c, b, n, n_head, n_kv, hd)
+        bound = 2.0 ** -8 * np.abs(want) * (1 + 2.0 ** -8) + 2.0 ** -16 * size.max()
+        assert (np.abs(new[b] - want) <= bound).all(), np.abs(new[b] - want).max()
+        assert (np.abs(new[b] - general[b]) <= 2 * bound).all()
+
+
+@pytest.mark.parametrize("what", ["q", "sk", "sv", "large"])
+def test_infinities_and_the_largest_values(what):
+    """One infinite input, and value scales near the end of the 32-bit range: the same finite results, infinities and
+    invalid values as the general kernel's."""
+    def edit(c):
+        if what == "q":
+            c["q"][0, 5] = np.inf
+        elif what == "large":
+            c["sv"][0, 3, 0] = 2e36
+        else:
+            c[what][0, 3, 0] = np.inf
+    _, (new, general) = both(8, 2, 128, (40, 20), seed=3, edit=edit)
+    assert np.array_equal(np.isfinite(new), np.isfinite(general))
+    fine = np.isfinite(new)
+    # bf16 neighbours at most
+    assert (np.abs(new[fine] - general[fine]) <= 2.0 ** -7 * np.abs(general[fine]) + 1e-4).all()
+    assert np.array_equal(np.sign(new[~fine]), np.sign(general[~fine]))

@@ -16,6 +16,8 @@
 // rounding (different reduction trees, accurate sincosf instead of the fast
 // intrinsic); tests/test_gpu_step.py states the tolerances.
 #include "common.cuh"
+#include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <mutex>
 
@@ -260,6 +262,8 @@ struct AttnParams {
     float scale;
     int score_stride;           // floats between the score rows of two query heads in shared memory
     int nsplit;                 // CTAs (= cluster size) that share the positions of one (kv head, sequence)
+    int t_limit;                // positions a launch may read, whatever `positions` holds
+    int stages;                 // attention_mma_kernel: chunks of a warp's ring in shared memory
 };
 
 constexpr int kAttnThreads = 256;
@@ -301,7 +305,7 @@ attention_kernel(const __grid_constant__ AttnParams P)
     const int kvh = blockIdx.x, seq = blockIdx.y, split = blockIdx.z, nsplit = P.nsplit;
     const int hd = P.head_dim;
     const int Tw = P.positions ? P.positions[seq] + 1 : P.seq_len;
-    const int T = Tw < P.score_stride * nsplit ? Tw : P.score_stride * nsplit;   // never past what this launch was sized for
+    const int T = Tw < P.t_limit ? Tw : P.t_limit;                 // never past what this launch was sized for
     const int per = (T + nsplit - 1) / nsplit;
     const int t_lo = split * per, t_hi = t_lo + per < T ? t_lo + per : T;       // this CTA's positions
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -506,6 +510,378 @@ attention_kernel(const __grid_constant__ AttnParams P)
 }
 
 // ---------------------------------------------------------------------------
+// The same attention on the tensor cores, for head_dim 64 / 96 / 128 and 16-byte aligned caches.
+// Bound: the cache, 2 * head_dim + 8 bytes a position and kv head (11 clocks of an SM's share of HBM at head_dim 128).
+// The kernel above needs ~60 clocks for them (an int8 -> float conversion per element on the quarter-rate pipe, a
+// multiply-add per element and query head, the shuffles of the dot products): 0.8 TB/s at 24 sequences of 2-4 k
+// positions, 195 us.  Here both products are mma.m16n8k16 with the cache as the B operand, one kv head's query heads in
+// the A rows, and nothing is rounded on the way: an int8 is exact in bf16, and a 32-bit q (or softmax weight times value
+// scale) is cut into three bf16 pieces of 8 significant bits, which are exact together.  With up to four query heads
+// the pieces sit in rows 0-3, 4-7 and 8-11 of one MMA; with eight, in rows 0-7 and 8-15 of one and rows 0-7 of a second.
+// A warp walks chunks of 16 positions with a running maximum; cp.async keeps two or three chunks (8-12 KB) in flight per
+// warp, sixteen warps per SM (128 registers: q is read from shared memory again for every chunk; with q in registers
+// twelve warps were resident: 31 against 30 us on 256 x 192 positions, 51 against 53 on 24 x 4096).  The partial results
+// of a CTA's warps meet in shared memory, those of a cluster's CTAs over distributed shared memory as above.
+// Measured, 32/8 heads of 128: 24 sequences of 2-4 k positions 195 -> 53 us (3.0 TB/s); bound now by instruction issue
+// (about 600 instructions a chunk, the ALU pipe half busy with the int8 conversions) and the CTAs' dependent start.
+// ---------------------------------------------------------------------------
+constexpr int kMmaWarps = 8;             // most warps of a CTA
+constexpr int kMmaPos = 16;              // positions of a chunk
+constexpr int kMmaStages = 3;
+constexpr int kMmaHeads = 8;             // most query heads per kv head
+__host__ __device__ constexpr int mma_stage_bytes(int hd) { return 2 * kMmaPos * hd + 2 * kMmaPos * 4; }   // K, V, scales
+// A warp's weighted values in shared memory: the kHD / 8 consecutive dims that a lane holds of a column, padded so that
+// the 16-byte stores of a quarter warp (two heads, four columns two apart) meet different banks.
+__host__ __device__ constexpr int mma_acc_col(int hd) { return hd == 64 ? 12 : 20; }
+__host__ __device__ constexpr int mma_acc_row(int hd) { return 8 * mma_acc_col(hd) + 4; }
+__host__ __device__ constexpr int mma_smem_bytes(int hd, int warps, int stages, int heads)
+{
+    return warps * stages * mma_stage_bytes(hd) + (2 * kMmaWarps + 2) * kMmaHeads * 4 + 3 * heads * (hd / 4 + 1) * 8;
+}
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ float exp2_approx(float x)
+{
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// int8 in the low byte of each half of x (the high bytes are ignored) -> two bf16, exact:
+// the seven magnitude bits above 128, minus 128, or minus 256 where the sign bit is set.
+__device__ __forceinline__ uint32_t s8_pair_to_bf16(uint32_t x)
+{
+    uint32_t v;
+    const uint32_t mag = and_or(x, 0x007F007Fu, 0x43004300u), off = and_or(x, 0x00800080u, 0xC300C300u);
+    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(v) : "r"(mag), "r"(off));
+    return v;
+}
+// x = hi + mid + lo, each with at most 8 significant bits (in the upper half of a register).  An infinity stays in hi
+// alone; a NaN stays a NaN in hi whatever its payload.
+__device__ __forceinline__ void split_bf16x3(float x, float& hi, float& mid, float& lo)
+{
+    const uint32_t u = __float_as_uint(x);
+    hi = __uint_as_float(x == x ? u & 0xFFFF0000u : 0x7FFF0000u);
+    const float r = hi == x ? 0.f : x - hi;
+    mid = __uint_as_float(__float_as_uint(r) & 0xFFFF0000u);
+    lo = r == mid ? 0.f : r - mid;
+}
+// the upper halves of two registers as one bf16 pair (a in the low half)
+__device__ __forceinline__ uint32_t pack_hi16(float a, float b) { return prmt(__float_as_uint(a), __float_as_uint(b), 0x7632u); }
+
+// the same for the product of two floats, whose NaN the hardware makes canonical
+__device__ __forceinline__ void split_product_bf16x3(float x, float& hi, float& mid, float& lo)
+{
+    hi = __uint_as_float(__float_as_uint(x) & 0xFFFF0000u);
+    const float r = hi == x ? 0.f : x - hi;
+    mid = __uint_as_float(__float_as_uint(r) & 0xFFFF0000u);
+    lo = r - mid;
+}
+
+template <int kHD, bool kWide>           // kWide: eight query heads per kv head, else up to four
+__global__ void __launch_bounds__(kMmaWarps * 32, 2)
+attention_mma_kernel(const __grid_constant__ AttnParams P)
+{
+    constexpr int kSteps = kHD / 16;     // MMA steps of the QK product
+    constexpr int kTiles = kHD / 8;      // MMA column tiles of the PV product = dims per lane group
+    constexpr int kRowPieces = kHD / 16; // 16-byte pieces of a cache row
+    constexpr int kStage = mma_stage_bytes(kHD);
+    extern __shared__ __align__(16) uint8_t mma_smem[];
+    const int nwarps = blockDim.x >> 5;
+    float* part_stats = reinterpret_cast<float*>(mma_smem + nwarps * P.stages * kStage);   // [warp][max, sum][head]
+    float* stats = part_stats + 2 * kMmaWarps * kMmaHeads;                                      // the CTA's [max, sum][head]
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int kvh = blockIdx.x, seq = blockIdx.y, split = blockIdx.z, nsplit = P.nsplit;
+    const int gqa = kWide ? 8 : P.n_head / P.n_head_kv;
+    const int Tw = P.positions ? P.positions[seq] + 1 : P.seq_len;
+    const int T = Tw < P.t_limit ? Tw : P.t_limit;
+    const int per = ((T + nsplit - 1) / nsplit + kMmaPos - 1) & ~(kMmaPos - 1);
+    const int t_lo = split * per, t_hi = t_lo + per < T ? t_lo + per : T;       // this CTA's positions
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+    const size_t kv_dim = (size_t)P.n_head_kv * kHD;
+    const int8_t* kc = P.kc + (size_t)seq * P.kv_stride + (size_t)kvh * kHD;
+    const int8_t* vc = P.vc + (size_t)seq * P.kv_stride + (size_t)kvh * kHD;
+    const float* scales = (lane < kMmaPos ? P.sk : P.sv) + (size_t)seq * (P.kv_stride / kHD) + kvh;
+    const float* q = P.q + ((size_t)seq * P.n_head + (size_t)kvh * gqa) * kHD;
+    // P.stages < kMmaStages: no warp has more chunks than that, and every chunk keeps a stage of its own
+    const int ring_bytes = P.stages * kStage;
+    uint8_t* ring = mma_smem + warp * ring_bytes;
+    const uint32_t ring_s = smem_addr(ring);
+
+    // A chunk in shared memory: K rows, V rows, 16 + 16 scales.  The 16-byte pieces of a row are permuted so that the
+    // lanes of a load phase meet different banks: K is read four pieces of two neighbouring rows at a time, V two (one
+    // and a half) pieces of four rows that lie two apart.
+    auto k_piece = [](int r, int c) { return kHD == 128 ? c ^ ((r & 1) << 2) : c; };
+    auto v_piece = [](int r, int c) { return kHD == 128 ? c ^ (((r >> 1) & 3) << 1) : kHD == 64 ? c ^ (((r >> 1) & 1) << 1) : c; };
+    const int first = t_lo + warp * kMmaPos, stride = nwarps * kMmaPos;
+    const int n = first < t_hi ? (t_hi - first + stride - 1) / stride : 0;      // this warp's chunks
+    // what a lane copies of a chunk: pieces of rows row0[j], the same in every chunk
+    uint32_t src_off[kRowPieces / 2], dst_k[kRowPieces / 2], dst_v[kRowPieces / 2];
+#pragma unroll
+    for (int j = 0; j < kRowPieces / 2; j++) {
+        const int p = j * 32 + lane, r = p / kRowPieces, c = p - r * kRowPieces;
+        src_off[j] = (uint32_t)r * (uint32_t)kv_dim + c * 16;
+        dst_k[j] = r * kHD + k_piece(r, c) * 16;
+        dst_v[j] = (kMmaPos + r) * kHD + v_piece(r, c) * 16;
+    }
+    const int8_t* k_next = kc + (size_t)first * kv_dim;
+    const int8_t* v_next = vc + (size_t)first * kv_dim;
+    const float* s_next = scales + (size_t)first * P.n_head_kv;
+    const uint32_t s_off = (uint32_t)(lane & (kMmaPos - 1)) * P.n_head_kv;
+    auto fetch = [&](int i) {
+        if (i < n) {
+            const int left = t_hi - (first + i * stride);          // positions of this chunk, 16 or more except in the last
+            const uint32_t dst = ring_s + (uint32_t)(i % kMmaStages) * kStage;
+            if (left >= kMmaPos) {
+#pragma unroll
+                for (int j = 0; j < kRowPieces / 2; j++) {
+                    cp_async16(dst + dst_k[j], k_next + src_off[j]);
+                    cp_async16(dst + dst_v[j], v_next + src_off[j]);
+                }
+                cp_async4(dst + 2 * kMmaPos * kHD + lane * 4, s_next + s_off);
+            } else {                                               // rows past the end: the last one again
+#pragma unroll
+                for (int j = 0; j < kRowPieces / 2; j++) {
+                    const int r = (j * 32 + lane) / kRowPieces;
+                    const uint32_t off = src_off[j] - (r < left ? 0u : (uint32_t)(r - left + 1) * (uint32_t)kv_dim);
+                    cp_async16(dst + dst_k[j], k_next + off);
+                    cp_async16(dst + dst_v[j], v_next + off);
+                }
+                const int r = lane & (kMmaPos - 1);
+                cp_async4(dst + 2 * kMmaPos * kHD + lane * 4, s_next + (r < left ? r : left - 1) * P.n_head_kv);
+            }
+            k_next += (size_t)stride * kv_dim; v_next += (size_t)stride * kv_dim; s_next += stride * P.n_head_kv;
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int i = 0; i < kMmaStages - 1; i++) fetch(i);
+
+    // q as A operand, cut once per CTA: pieces[piece][head][four dims], the four in the order 0, 2, 1, 3 (the bytes that
+    // one mask of a cache word leaves side by side).  MMA step s, lane t4 stands for four consecutive dims.
+    constexpr int kHeads = kWide ? 8 : 4;
+    uint2* pieces = reinterpret_cast<uint2*>(stats + 2 * kMmaHeads);
+    constexpr int kPieceRow = kHD / 4 + 1;                         // one more: the rows of a load phase on different banks
+    for (int i = threadIdx.x; i < kHeads * kHD / 4; i += blockDim.x) {
+        float hi[4], mid[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) split_bf16x3(i * 4 < gqa * kHD ? q[i * 4 + e] : 0.f, hi[e], mid[e], lo[e]);
+        uint2* at = pieces + i / (kHD / 4) * kPieceRow + i % (kHD / 4);
+        at[0] = make_uint2(pack_hi16(hi[0], hi[2]), pack_hi16(hi[1], hi[3]));
+        at[kHeads * kPieceRow] = make_uint2(pack_hi16(mid[0], mid[2]), pack_hi16(mid[1], mid[3]));
+        at[2 * kHeads * kPieceRow] = make_uint2(pack_hi16(lo[0], lo[2]), pack_hi16(lo[1], lo[3]));
+    }
+    __syncthreads();
+    const int head = kWide ? g : g & 3;                            // query head of this lane's rows (g and g + 8)
+    const uint2* q_row = pieces + head * kPieceRow + (kHD == 96 ? t4 * 2 : t4 * 4) + (kWide || g < 4 ? 0 : kHeads * kPieceRow);
+    const float to_log2 = P.scale * 1.4426950408889634f;           // weights are powers of two of the scaled scores
+
+    float acc[kTiles][4];
+#pragma unroll
+    for (int j = 0; j < kTiles; j++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc[j][e] = 0.f;
+    float m = -1e30f, l = 0.f;
+#pragma unroll 1
+    for (int i = 0; i < n; i++) {
+        cp_async_wait<kMmaStages - 2>();
+        __syncwarp();                                              // this chunk has landed; the one before has been read
+        fetch(i + kMmaStages - 1);
+        const uint8_t* K = ring + (i % kMmaStages) * kStage;
+        const uint8_t* V = K + kMmaPos * kHD;
+        const float* sc = reinterpret_cast<const float*>(V + kMmaPos * kHD);
+        const int t0 = first + i * stride + 2 * t4;                // this lane's positions: t0 + 8 u + {0, 1}
+        float w[2][2];
+        float mx = -1e30f;
+        uint32_t kw[2][kSteps];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int r = u * 8 + g;
+            if (kHD == 96) {
+#pragma unroll
+                for (int b = 0; b < 3; b++) {
+                    const uint2 x = *reinterpret_cast<const uint2*>(K + r * kHD + b * 32 + t4 * 8);
+                    kw[u][2 * b] = x.x; kw[u][2 * b + 1] = x.y;
+                }
+            } else {
+#pragma unroll
+                for (int b = 0; b < kSteps / 4; b++) {
+                    const uint4 x = *reinterpret_cast<const uint4*>(K + r * kHD + k_piece(r, b * 4 + t4) * 16);
+                    kw[u][4 * b] = x.x; kw[u][4 * b + 1] = x.y; kw[u][4 * b + 2] = x.z; kw[u][4 * b + 3] = x.w;
+                }
+            }
+        }
+        // q is read again for every chunk: its 32 registers would cost a quarter of the resident warps
+        float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int s = 0; s < kSteps; s++) {
+            const uint2* at = q_row + (kHD == 96 ? (s >> 1) * 8 + (s & 1) : (s >> 2) * 16 + (s & 3));
+            const uint2 x0 = at[0];
+            const uint2 x1 = kWide ? at[kHeads * kPieceRow] : g < 4 ? at[2 * kHeads * kPieceRow] : make_uint2(0u, 0u);
+            const uint2 x2 = kWide ? at[2 * kHeads * kPieceRow] : make_uint2(0u, 0u);
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const uint32_t b0 = s8_pair_to_bf16(kw[u][s]), b1 = s8_pair_to_bf16(kw[u][s] >> 8);
+                mma_bf16_16816(c[u], x0.x, x1.x, x0.y, x1.y, b0, b1);
+                if (kWide) mma_bf16_16816(c[u], x2.x, 0u, x2.y, 0u, b0, b1);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                float x = c[u][e] + c[u][2 + e];
+                if (!kWide) x += __shfl_xor_sync(0xFFFFFFFFu, x, 16);
+                x *= sc[u * 8 + 2 * t4 + e] * to_log2;
+                w[u][e] = x;
+                if (t0 + u * 8 + e < t_hi) mx = fmaxf(mx, x);
+            }
+        }
+        mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 2));
+        // Weights are 2^(score - m) with m at least the maximum so far; it is set six above a new maximum, so that the
+        // sums are rarely rescaled.
+        if (__any_sync(0xFFFFFFFFu, mx > m)) {
+            const float mn = mx > m ? mx + 6.f : m, f = exp2_approx(m - mn);
+            m = mn;
+            if (i > 0) {
+                l *= f;
+#pragma unroll
+                for (int j = 0; j < kTiles; j++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) acc[j][e] *= f;
+            }
+        }
+        uint32_t ap[4], apl[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            float hi[2], mid[2], lo[2];
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const bool live = t0 + u * 8 + e < t_hi;
+                const float p = live ? exp2_approx(w[u][e] - m) : 0.f;
+                l += p;
+                split_product_bf16x3(live ? p * sc[kMmaPos + u * 8 + 2 * t4 + e] : 0.f, hi[e], mid[e], lo[e]);
+            }
+            if (kWide) {
+                ap[2 * u] = pack_hi16(hi[0], hi[1]); ap[2 * u + 1] = pack_hi16(mid[0], mid[1]);
+                apl[u] = pack_hi16(lo[0], lo[1]);
+            } else {
+                ap[2 * u] = g < 4 ? pack_hi16(hi[0], hi[1]) : pack_hi16(mid[0], mid[1]);
+                ap[2 * u + 1] = g < 4 ? pack_hi16(lo[0], lo[1]) : 0u;
+            }
+        }
+        // column g of value tile j stands for dim kTiles * g + j
+        uint32_t vw[4][kTiles / 4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int r = 2 * t4 + (e & 1) + (e >> 1) * 8;
+            if (kHD == 128) {
+                const uint4 x = *reinterpret_cast<const uint4*>(V + r * kHD + v_piece(r, g) * 16);
+                vw[e][0] = x.x; vw[e][1] = x.y; vw[e][kTiles / 4 - 2] = x.z; vw[e][kTiles / 4 - 1] = x.w;
+            } else if (kHD == 64) {
+                const uint2 x = *reinterpret_cast<const uint2*>(V + r * kHD + v_piece(r, g >> 1) * 16 + (g & 1) * 8);
+                vw[e][0] = x.x; vw[e][1] = x.y;
+            } else {
+#pragma unroll
+                for (int b = 0; b < kTiles / 4; b++) vw[e][b] = *reinterpret_cast<const uint32_t*>(V + r * kHD + g * kTiles + b * 4);
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < kTiles / 4; b++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {                          // dims 4 b + 2 h and the next: halves {row, row + 1}
+                const uint32_t sel = h ? 0x7632u : 0x5410u;
+                const uint32_t x0 = prmt(vw[0][b], vw[1][b], sel), x1 = prmt(vw[2][b], vw[3][b], sel);
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const uint32_t b0 = s8_pair_to_bf16(e ? x0 >> 8 : x0), b1 = s8_pair_to_bf16(e ? x1 >> 8 : x1);
+                    float (&c)[4] = acc[4 * b + 2 * h + e];
+                    mma_bf16_16816(c, ap[0], ap[1], ap[2], ap[3], b0, b1);
+                    if (kWide) mma_bf16_16816(c, apl[0], 0u, apl[1], 0u, b0, b1);
+                }
+            }
+    }
+    cp_async_wait<0>();
+    __syncwarp();                                                  // the ring is the warp's own: its partial result goes there
+    l += __shfl_xor_sync(0xFFFFFFFFu, l, 1);
+    l += __shfl_xor_sync(0xFFFFFFFFu, l, 2);
+    float* mine = reinterpret_cast<float*>(ring);                  // [head][column], padded: see mma_acc_index
+    const bool owner = kWide || (g < 4 && head < gqa);
+#pragma unroll
+    for (int j = 0; j < kTiles; j += 4)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            float x[4];
+#pragma unroll
+            for (int d = 0; d < 4; d++) {
+                x[d] = acc[j + d][e] + acc[j + d][2 + e];
+                if (!kWide) x[d] += __shfl_xor_sync(0xFFFFFFFFu, x[d], 16);
+            }
+            if (owner) *reinterpret_cast<float4*>(mine + head * mma_acc_row(kHD) + (2 * t4 + e) * mma_acc_col(kHD) + j) = make_float4(x[0], x[1], x[2], x[3]);
+        }
+    if (owner && t4 == 0) {
+        part_stats[(2 * warp) * kMmaHeads + head] = m;
+        part_stats[(2 * warp + 1) * kMmaHeads + head] = l;
+    }
+    __syncthreads();
+    // the CTA's sums over its warps, four dims a thread, in place in the first warp's ring
+    float* accs = reinterpret_cast<float*>(mma_smem);
+    const int ring_floats = ring_bytes / 4;
+    int16_t* out = P.out + ((size_t)seq * P.n_head + (size_t)kvh * gqa) * kHD;
+    for (int i = threadIdx.x; i < gqa * kHD / 4; i += blockDim.x) {
+        const int h = i / (kHD / 4), d = (i - h * (kHD / 4)) * 4, at = h * mma_acc_row(kHD) + d / kTiles * mma_acc_col(kHD) + d % kTiles;
+        float mm = -1e30f, den = 0.f;
+        float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int wv = 0; wv < nwarps; wv++) mm = fmaxf(mm, part_stats[2 * wv * kMmaHeads + h]);
+        for (int wv = 0; wv < nwarps; wv++) {
+            const float f = exp2_approx(part_stats[2 * wv * kMmaHeads + h] - mm);   // a warp without positions: 0
+            const float4 x = *reinterpret_cast<const float4*>(accs + wv * ring_floats + at);
+            num.x += f * x.x; num.y += f * x.y; num.z += f * x.z; num.w += f * x.w;
+            den += f * part_stats[(2 * wv + 1) * kMmaHeads + h];
+        }
+        if (nsplit == 1) {
+            const uint32_t lo = (uint16_t)float_to_bf16_rne(num.x / den) | (uint32_t)(uint16_t)float_to_bf16_rne(num.y / den) << 16;
+            const uint32_t hi = (uint16_t)float_to_bf16_rne(num.z / den) | (uint32_t)(uint16_t)float_to_bf16_rne(num.w / den) << 16;
+            int16_t* o = out + i * 4;
+            if ((reinterpret_cast<uintptr_t>(o) & 7) == 0) {
+                *reinterpret_cast<uint2*>(o) = make_uint2(lo, hi);
+            } else {
+                o[0] = (int16_t)lo; o[1] = (int16_t)(lo >> 16); o[2] = (int16_t)hi; o[3] = (int16_t)(hi >> 16);
+            }
+        } else {
+            *reinterpret_cast<float4*>(accs + at) = num;           // read above by this thread only
+            if (d == 0) { stats[h] = mm; stats[kMmaHeads + h] = den; }
+        }
+    }
+    if (nsplit == 1) return;
+    // ---- merge the slices of the cluster: rank r finishes the output elements r * threads, ...
+    cluster_barrier();
+    for (int i = split * blockDim.x + threadIdx.x; i < gqa * kHD; i += nsplit * blockDim.x) {
+        const int h = i / kHD, d = i - h * kHD, at = h * mma_acc_row(kHD) + d / kTiles * mma_acc_col(kHD) + d % kTiles;
+        float mm = -1e30f;
+        for (int r = 0; r < nsplit; r++) mm = fmaxf(mm, ld_dsmem_f32(dsmem_addr(stats + h, r)));
+        float num = 0.f, den = 0.f;
+        for (int r = 0; r < nsplit; r++) {
+            const float f = exp2_approx(ld_dsmem_f32(dsmem_addr(stats + h, r)) - mm);   // an empty slice has max -1e30: weight 0
+            num += f * ld_dsmem_f32(dsmem_addr(accs + at, r));
+            den += f * ld_dsmem_f32(dsmem_addr(stats + kMmaHeads + h, r));
+        }
+        out[i] = float_to_bf16_rne(num / den);
+    }
+    cluster_barrier();                                             // nobody reads this CTA's shared memory any more
+}
+
+// ---------------------------------------------------------------------------
 // Greedy argmax, one CTA per sequence.  Ties resolve as in the engine's kernel
 // (engine/kernels.hip:90-122: 256 threads scan i = tid, tid + 256, ... with a
 // strict ">", then a halving tree in which slot t meets slot t + s and keeps its
@@ -636,6 +1012,48 @@ static int rope_kv_launch(RopeKvParams& P, float theta, int batch, void* stream,
     return launch(rope_kv_kernel, dim3(ctas, batch), dim3(threads), 0, stream, who, Q, F);
 }
 
+// Launches attention_mma_kernel when it takes the shape (returns its status, 0 or negative), else returns 1.
+// It takes head_dim 64 / 96 / 128 with rows of the caches on 16-byte boundaries.
+static int attention_mma_launch(AttnParams P, int gqa, int max_len, int batch, void* stream, const char* who)
+{
+    const int hd = P.head_dim;
+    if ((hd != 64 && hd != 96 && hd != 128) || P.kv_stride % 16 != 0 ||
+        ((reinterpret_cast<uintptr_t>(P.kc) | reinterpret_cast<uintptr_t>(P.vc)) & 15) != 0)
+        return 1;
+    // Slices while three CTAs per SM (four are resident) are not there, of 64 positions or more: a CTA costs ~6 us of
+    // dependent loads and merging whatever its length.  32/8 heads of 128, us with 1 / 2 / 4 / 8 slices: 24 sequences of
+    // 4096 77 / 67 / 53 / 53; 64 of 1000 36 / 37 / 42 / 60; 256 of 192 30 / 53 / 84 / 168; one of 8000 100 / 54 / 29 / 17.
+    int nsplit = 1;
+    const long long pairs = (long long)P.n_head_kv * batch;
+    while (nsplit < 8 && pairs * nsplit < 3ll * sm_count() && max_len / (nsplit * 2) >= 64) nsplit *= 2;
+    P.nsplit = nsplit;
+    // Eight warps instead of four where all CTAs are resident at once even so: one sequence of 8000 positions
+    // 16.9 -> 13.9 us, four of them with 64 query heads 34 -> 26 us; otherwise (256 of 192: 30 -> 41 us) or with two
+    // chunks a warp or fewer the larger CTA only waits longer.
+    const int warps = pairs * nsplit <= 2ll * sm_count() && max_len / nsplit >= 256 ? 8 : 4;
+    typedef void (*Kern)(const AttnParams);
+    static const Kern table[3][2] = {{attention_mma_kernel<64, false>, attention_mma_kernel<64, true>},
+                                     {attention_mma_kernel<96, false>, attention_mma_kernel<96, true>},
+                                     {attention_mma_kernel<128, false>, attention_mma_kernel<128, true>}};
+    const int hi = hd == 64 ? 0 : hd == 96 ? 1 : 2, wi = gqa == 8 ? 1 : 0;
+    Kern kern = table[hi][wi];
+    // short contexts keep little shared memory: the projections' kernels either side hold most of an SM's, and this
+    // kernel starts early only beside them
+    const int per = ((P.t_limit + nsplit - 1) / nsplit + kMmaPos - 1) / kMmaPos;
+    const int least = (gqa * mma_acc_row(hd) * 4 + mma_stage_bytes(hd) - 1) / mma_stage_bytes(hd);   // the partial result's room
+    P.stages = std::min(kMmaStages, std::max(least, (per + warps - 1) / warps));
+    const int smem = mma_smem_bytes(hd, warps, P.stages, gqa == 8 ? 8 : 4);
+    static std::atomic<bool> attr_set[64][3][2];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !attr_set[dev][hi][wi].load(std::memory_order_relaxed)) {
+        const int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, mma_smem_bytes(hd, kMmaWarps, kMmaStages, gqa == 8 ? 8 : 4)), who);
+        if (rc) return rc;
+        if (dev >= 0 && dev < 64) attr_set[dev][hi][wi].store(true, std::memory_order_relaxed);
+    }
+    return launch_clustered_z(kern, dim3(P.n_head_kv, batch, nsplit), dim3(warps * 32), (size_t)smem, stream, who, nsplit, P);
+}
+
 static int attention_launch(AttnParams& P, int max_len, int batch, void* stream, const char* who)
 {
     if (P.head_dim < 4 || P.head_dim > 256 || (P.head_dim & 3) || P.n_head_kv < 1 || P.n_head < P.n_head_kv ||
@@ -659,6 +1077,9 @@ static int attention_launch(AttnParams& P, int max_len, int batch, void* stream,
     P.score_stride = (per + 3) & ~3;
     const size_t smem = smem_for(nsplit);
     if (smem > 200 * 1024) return fail(S12_ERR_TOO_LARGE, "%s: seq_len %d needs more shared memory than one CTA has", who, max_len);
+    P.t_limit = P.score_stride * nsplit;
+    const int mma = attention_mma_launch(P, gqa, max_len, batch, stream, who);
+    if (mma <= 0) return mma;
     typedef void (*Kern)(const AttnParams);
     static const Kern table[4][2] = {{attention_kernel<1, 1>, attention_kernel<1, 2>}, {attention_kernel<2, 1>, attention_kernel<2, 2>},
                                      {attention_kernel<4, 1>, attention_kernel<4, 2>}, {attention_kernel<8, 1>, attention_kernel<8, 2>}};
