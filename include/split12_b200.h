@@ -369,10 +369,23 @@ int s12_pack_find_base_exp_host(const uint64_t* hist256);
 int s12_pack_async(const void* bf16, int M, int K, int base_exp, void* sm, void* gr,
                    void* row_off, void* stream);
 
+/* Histogram, window search and first pass as one call without the host between
+ * them: meta (device, int32 [2]) receives base_exp and the number of escapes,
+ * which the caller reads back once; same bytes as the three calls above.
+ * scratch: S12_PACK_SCRATCH_BYTES on the device, 8-byte aligned, free again when
+ * the call's kernels have run.  M and K at least 1. */
+#define S12_PACK_SCRATCH_BYTES (257 * 8)
+int s12_pack_auto_async(const void* bf16, int M, int K, void* scratch, void* meta, void* sm, void* gr,
+                        void* row_off, void* stream);
+
 /* Second pass (split12_pack.c:106-124): cols / correct / wrong in ascending
  * column order within each row. */
 int s12_pack_fill_async(const void* bf16, int M, int K, int base_exp, const void* row_off,
                         void* cols, void* correct, void* wrong, void* stream);
+/* The same from the first pass's gr: finds the escapes in its zero nibbles (a
+ * quarter of the bytes) and reads only their values from bf16. */
+int s12_pack_fill_groups_async(const void* bf16, const void* gr, int M, int K, int base_exp,
+                               const void* row_off, void* cols, void* correct, void* wrong, void* stream);
 
 /* --------------------------------------------------------------------------
  * The decode step around the projections (engine/kernels.hip)

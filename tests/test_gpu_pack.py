@@ -62,3 +62,47 @@ def test_pack_under_dependent_launch(O, golden):
             _check(CompressedWeight.pack_on_device(dev(w)), O.pack(w))
     finally:
         eng.set_dependent_launch(old)
+
+
+@pytest.mark.parametrize("M,K,frac", [(1, 2, 1.0), (5, 6, 0.5), (3, 8, 0.3), (7, 24, 0.2), (2, 1032, 0.1), (3, 4104, 1e-2), (1, 16384, 0.9),
+                                      (1023, 16, 0.2), (8191, 8, 0.1), (8192, 34, 0.05), (8193, 16, 0.1), (20000, 40, 0.02)])
+@pytest.mark.parametrize("offset", [0, 1, 8])
+def test_edges_of_the_passes(O, M, K, frac, offset):
+    """Rows around the scan's 8192, columns around the fill's 256 and 1024, values off a 16-byte boundary (offset
+    elements into a buffer): one call, and the separate passes on the same values."""
+    from turbo_lossless_b200 import CompressedWeight, capi
+    from turbo_lossless_b200.capi import check
+    rng = np.random.default_rng(M + K)
+    w = O.synth_weights(M, K, M + K, outlier_frac=0.0)
+    w = np.where(rng.random((M, K)) < frac, rng.integers(0, 1 << 16, (M, K), dtype=np.uint16), w)   # any exponent
+    ref = O.pack(w)
+    room = torch.zeros(M * K + 16, dtype=torch.int16, device="cuda")
+    wd = room[offset:offset + M * K].view(M, K)
+    wd.copy_(dev(w))
+    _check(CompressedWeight.pack_on_device(wd), ref)
+    _check(CompressedWeight.pack_on_device(wd, base_exp=ref.base_exp), ref)
+    lib = capi.load()
+    hist = torch.empty(256, dtype=torch.int64, device="cuda")
+    check(lib.s12_pack_histogram_async(wd.data_ptr(), M * K, hist.data_ptr(), None))
+    assert np.array_equal(hist.cpu().numpy(), np.bincount((w.reshape(-1) >> 7) & 0xFF, minlength=256))
+    if ref.num_patches:
+        got = [torch.zeros(ref.num_patches, dtype=d, device="cuda") for d in (torch.int32, torch.int16, torch.int16)]
+        check(lib.s12_pack_fill_async(wd.data_ptr(), M, K, ref.base_exp, dev(ref.row_off).data_ptr(), *[t.data_ptr() for t in got], None))
+        for t, a in zip(got, (ref.cols, ref.correct, ref.wrong)):
+            assert np.array_equal(t.cpu().numpy(), a)
+
+
+@pytest.mark.parametrize("base_exp", [-1, 0, 100, 112, 239, 240, 241, 254, -9])
+def test_given_window_over_every_value(O, base_exp):
+    """All 65536 bf16 patterns (their sixteen-element chunks hold neighbouring exponents) with a window given by the caller."""
+    from turbo_lossless_b200 import CompressedWeight
+    w = np.random.default_rng(1).permutation(np.arange(1 << 16, dtype=np.uint32)).astype(np.uint16).reshape(256, 256)
+    cw = CompressedWeight.pack_on_device(dev(w), base_exp=base_exp)
+    e = ((w >> 7) & 0xFF).astype(np.int32) - base_exp
+    grp = np.where((e >= 1) & (e <= 15), e, 0).astype(np.uint8).reshape(-1)
+    assert np.array_equal(cw.split_sm.cpu().numpy(), (((w >> 15) << 7) | (w & 0x7F)).astype(np.uint8).reshape(-1))
+    assert np.array_equal(cw.split_gr.cpu().numpy(), grp[0::2] | (grp[1::2] << 4))
+    rows, cols = np.nonzero(grp.reshape(w.shape) == 0)
+    assert cw.num_patches == len(cols) and np.array_equal(cw.patch_cols.cpu().numpy(), cols)
+    assert np.array_equal(cw.row_offsets.cpu().numpy(), np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=256))]))
+    assert np.array_equal(cw.patch_correct.cpu().numpy().view(np.uint16), w[rows, cols])

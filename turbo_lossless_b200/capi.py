@@ -65,6 +65,8 @@ SIGNATURES = {
     "s12_pack_histogram_async": (_i, [_vp, C.c_int64, _vp, _vp]),
     "s12_pack_find_base_exp_host": (_i, [_vp]),
     "s12_pack_async": (_i, [_vp, _i, _i, _i, _vp, _vp, _vp, _vp]),
+    "s12_pack_auto_async": (_i, [_vp, _i, _i] + [_vp] * 6),
+    "s12_pack_fill_groups_async": (_i, [_vp, _vp, _i, _i, _i] + [_vp] * 5),
     "s12_pack_fill_async": (_i, [_vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp]),
     "launch_embed_lookup": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp]),
     "launch_argmax": (_i, [_vp, _vp, _i, _vp]),

@@ -21,6 +21,8 @@ import torch
 from . import capi
 from .capi import S12PatchBatchDesc, S12Tensor, check
 
+PACK_SCRATCH_BYTES = 257 * 8               # S12_PACK_SCRATCH_BYTES of the header
+
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
@@ -138,24 +140,28 @@ class CompressedWeight:
         M, K = w.shape
         dev = w.device
         st = _stream()
-        if base_exp is None:
-            hist = torch.empty(256, dtype=torch.int64, device=dev)
-            check(lib.s12_pack_histogram_async(w.data_ptr(), M * K, hist.data_ptr(), st), "s12_pack_histogram_async")
-            h = np.ascontiguousarray(hist.cpu().numpy().astype(np.uint64))
-            base_exp = int(lib.s12_pack_find_base_exp_host(h.ctypes.data))
         sm = torch.empty(M * K, dtype=torch.uint8, device=dev)
         gr = torch.empty(M * K // 2, dtype=torch.uint8, device=dev)
         row_off = torch.empty(M + 1, dtype=torch.int32, device=dev)
-        check(lib.s12_pack_async(w.data_ptr(), M, K, base_exp, sm.data_ptr(), gr.data_ptr(), row_off.data_ptr(), st),
-              "s12_pack_async")
-        npat = int(row_off[-1].item())
+        if base_exp is None and M * K > 0:
+            # scratch for the histogram, then {base_exp, escapes}: one read by the host
+            tmp = torch.empty(PACK_SCRATCH_BYTES + 8, dtype=torch.uint8, device=dev)
+            meta = tmp[PACK_SCRATCH_BYTES:].view(torch.int32)
+            check(lib.s12_pack_auto_async(w.data_ptr(), M, K, tmp.data_ptr(), meta.data_ptr(), sm.data_ptr(), gr.data_ptr(),
+                                          row_off.data_ptr(), st), "s12_pack_auto_async")
+            base_exp, npat = meta.tolist()
+        else:
+            base_exp = -1 if base_exp is None else base_exp             # the window search's answer for an empty tensor
+            check(lib.s12_pack_async(w.data_ptr(), M, K, base_exp, sm.data_ptr(), gr.data_ptr(), row_off.data_ptr(), st),
+                  "s12_pack_async")
+            npat = int(row_off[-1].item())
         out = cls(M=M, K=K, base_exp=base_exp, split_sm=sm, split_gr=gr, num_patches=npat)
         if npat > 0:
             cols = torch.empty(npat, dtype=torch.int32, device=dev)
             correct = torch.empty(npat, dtype=torch.int16, device=dev)
             wrong = torch.empty(npat, dtype=torch.int16, device=dev)
-            check(lib.s12_pack_fill_async(w.data_ptr(), M, K, base_exp, row_off.data_ptr(), cols.data_ptr(),
-                                          correct.data_ptr(), wrong.data_ptr(), st), "s12_pack_fill_async")
+            check(lib.s12_pack_fill_groups_async(w.data_ptr(), gr.data_ptr(), M, K, base_exp, row_off.data_ptr(), cols.data_ptr(),
+                                                 correct.data_ptr(), wrong.data_ptr(), st), "s12_pack_fill_groups_async")
             out.row_offsets, out.patch_cols, out.patch_correct, out.patch_wrong = row_off, cols, correct, wrong
             if escape_table:
                 out.build_escape_table_on_device()
