@@ -262,24 +262,39 @@ struct EscCursor {
     uint32_t v0, v1;            // their exact bf16 bit patterns
 };
 constexpr int kNoEscape = 0x7FFFFFFF;
-// Index of the first entry of `row` with column >= kstart, and the end of the row's list.  Out of line (it
-// runs once per tile); the cursor itself is filled by the inlined caller so that it stays in registers.
-__device__ __noinline__ int2 esc_find(const int* __restrict__ row_off, const int* __restrict__ cols, int row, int kstart)
+// First entry in [a, b) with column >= kstart (b: none).  Seven columns are looked at together, so that a list of up to
+// seven entries takes one round of memory latency and one of up to 63 takes two.
+__device__ __noinline__ int esc_lower_bound(const int* __restrict__ cols, int a, int b, int kstart)
 {
-    int a = row_off[row], b = row_off[row + 1];
-    const int end = b;
-    while (a < b) { const int mid = (a + b) >> 1; if (cols[mid] < kstart) a = mid + 1; else b = mid; }
-    return make_int2(a, end);
+    while (a < b) {
+        const int step = (b - a + 7) >> 3;
+        int c[7];
+#pragma unroll
+        for (int i = 0; i < 7; i++) c[i] = a + (i + 1) * step - 1 < b ? cols[a + (i + 1) * step - 1] : kNoEscape;
+        int below = 0;                                            // looked-at entries below kstart: the first ones
+#pragma unroll
+        for (int i = 0; i < 7; i++) below += c[i] < kstart;
+        a += below * step;
+        if (below < 7 && a + step - 1 < b) b = a + step - 1;      // that entry was looked at: kstart or more
+    }
+    return a;
+}
+// Loads the entry at e.pos and the one after it.
+__device__ __forceinline__ void esc_load(EscCursor& e, const GemmTensor& T)
+{
+    e.c0 = e.c1 = kNoEscape; e.v0 = e.v1 = 0;
+    if (e.pos < e.end) { e.c0 = T.cols[e.pos]; e.v0 = (uint16_t)T.correct[e.pos]; }
+    if (e.pos + 1 < e.end) { e.c1 = T.cols[e.pos + 1]; e.v1 = (uint16_t)T.correct[e.pos + 1]; }
 }
 // Positions the cursor on the first entry of `row` with column >= kstart.
 __device__ __forceinline__ void esc_seek(EscCursor& e, const GemmTensor& T, int row, int kstart)
 {
-    e.pos = e.end = 0; e.c0 = e.c1 = kNoEscape; e.v0 = e.v1 = 0;
-    if (T.row_off == nullptr || row >= T.M) return;
-    const int2 pe = esc_find(T.row_off, T.cols, row, kstart);
-    e.pos = pe.x; e.end = pe.y;
-    if (e.pos < e.end) { e.c0 = T.cols[e.pos]; e.v0 = (uint16_t)T.correct[e.pos]; }
-    if (e.pos + 1 < e.end) { e.c1 = T.cols[e.pos + 1]; e.v1 = (uint16_t)T.correct[e.pos + 1]; }
+    e.pos = e.end = 0;
+    if (T.row_off != nullptr && row < T.M) {
+        e.pos = T.row_off[row]; e.end = T.row_off[row + 1];
+        if (kstart > 0) e.pos = esc_lower_bound(T.cols, e.pos, e.end, kstart);
+    }
+    esc_load(e, T);
 }
 __device__ __forceinline__ void esc_advance(EscCursor& e, const GemmTensor& T)
 {
@@ -295,13 +310,28 @@ __device__ __forceinline__ void esc_apply(EscCursor& e, const GemmTensor& T, int
         const int idx = e.c0 - k0;
         if (idx >= 0) {
             const uint32_t keep = (idx & 1) ? 0x0000FFFFu : 0xFFFF0000u, ins = (idx & 1) ? (e.v0 << 16) : e.v0;
-            // one predicated (v & keep) | ins per register: written as PTX so that the register array is
-            // not turned into an indexed local-memory array
+            // One predicated (v & keep) | ins per register of the quarter that holds the entry, behind a branch per
+            // quarter (a warp rarely has more than one entry at a time).  Written as PTX so that the register array
+            // is not turned into an indexed local-memory array.  With all 32 registers tested for every entry, the
+            // escapes cost a tenth of a launch at B = 64 and 0.015 % escapes (28672 x 4096: 47.4 us, 42.0 without them,
+            // 45.9 this way), and a fifth of the time of 14336 x 4096 experts with 0.25 % (whole block 740 -> 653 us).
             const int h = idx >> 1;
 #pragma unroll
-            for (int i = 0; i < 32; i++)
-                asm("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, %2;\n\t@p lop3.b32 %0, %0, %3, %4, 0xEA;\n\t}"
-                    : "+r"(v[i]) : "r"(h), "r"(i), "r"(keep), "r"(ins));
+            for (int q = 0; q < 4; q++)
+                asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\t"
+                             "shr.s32 t, %8, 3;\n\tsetp.ne.s32 p, t, %11;\n\t@p bra ESC_SKIP%=;\n\tand.b32 t, %8, 7;\n\t"
+                             "setp.eq.s32 p, t, 0;\n\t@p lop3.b32 %0, %0, %9, %10, 0xEA;\n\t"
+                             "setp.eq.s32 p, t, 1;\n\t@p lop3.b32 %1, %1, %9, %10, 0xEA;\n\t"
+                             "setp.eq.s32 p, t, 2;\n\t@p lop3.b32 %2, %2, %9, %10, 0xEA;\n\t"
+                             "setp.eq.s32 p, t, 3;\n\t@p lop3.b32 %3, %3, %9, %10, 0xEA;\n\t"
+                             "setp.eq.s32 p, t, 4;\n\t@p lop3.b32 %4, %4, %9, %10, 0xEA;\n\t"
+                             "setp.eq.s32 p, t, 5;\n\t@p lop3.b32 %5, %5, %9, %10, 0xEA;\n\t"
+                             "setp.eq.s32 p, t, 6;\n\t@p lop3.b32 %6, %6, %9, %10, 0xEA;\n\t"
+                             "setp.eq.s32 p, t, 7;\n\t@p lop3.b32 %7, %7, %9, %10, 0xEA;\n\t"
+                             "ESC_SKIP%=:\n\t}"
+                             : "+r"(v[8 * q]), "+r"(v[8 * q + 1]), "+r"(v[8 * q + 2]), "+r"(v[8 * q + 3]), "+r"(v[8 * q + 4]),
+                               "+r"(v[8 * q + 5]), "+r"(v[8 * q + 6]), "+r"(v[8 * q + 7])
+                             : "r"(h), "r"(keep), "r"(ins), "r"(q));
         }
         esc_advance(e, T);
     }
@@ -681,6 +711,7 @@ gemm_tc_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ CU
             if (lane == 0) mbar_arrive(b_rawempty + 8 * sr);      // this warp has read its share of the stage
             esc_apply(esc, T, kb * kBigK + gi * kTK, v);
             if (wo > 0) mbar_wait(b_free + 8 * gi, (wo - 1) & 1, P.status, 0x400u, &s_abort);
+            __syncwarp();                                         // lanes with escapes took another way
             tc_fence_after();
             tmem_st32(a_dst, v);
             tmem_st_wait();
