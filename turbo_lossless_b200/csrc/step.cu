@@ -34,31 +34,19 @@ __device__ __forceinline__ int16_t float_to_bf16_rne(float v)
     return (int16_t)((u + 0x7FFFu + ((u >> 16) & 1u)) >> 16);
 }
 
-// block-wide sum / max over up to 32 warps; every thread gets the result
-template <bool kMax>
-__device__ __forceinline__ float block_reduce(float v, float* scratch /* >= 33 floats */)
+// block-wide sum over up to 32 warps; every thread gets the result.  One barrier: every warp adds up the warps' sums
+// itself.  `scratch` serves one call of a kernel.
+__device__ __forceinline__ float block_sum(float v, float* scratch /* 32 floats */)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const float o = __shfl_xor_sync(0xFFFFFFFFu, v, off);
-        v = kMax ? fmaxf(v, o) : v + o;
-    }
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
     if (lane == 0) scratch[warp] = v;
     __syncthreads();
-    if (warp == 0) {
-        float w = lane < nwarps ? scratch[lane] : (kMax ? -INFINITY : 0.f);
+    float w = lane < nwarps ? scratch[lane] : 0.f;
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const float o = __shfl_xor_sync(0xFFFFFFFFu, w, off);
-            w = kMax ? fmaxf(w, o) : w + o;
-        }
-        if (lane == 0) scratch[32] = w;
-    }
-    __syncthreads();
-    const float r = scratch[32];
-    __syncthreads();                                              // scratch may be reused right away
-    return r;
+    for (int off = 16; off > 0; off >>= 1) w += __shfl_xor_sync(0xFFFFFFFFu, w, off);
+    return w;
 }
 
 // ---------------------------------------------------------------------------
@@ -82,36 +70,60 @@ embed_kernel(const int16_t* __restrict__ table, const int* __restrict__ tokens, 
 // RMSNorm -> bf16, optionally after x += residual written back in place
 // (engine/kernels.hip:355-393, 399-442).  One CTA per sequence.
 // ---------------------------------------------------------------------------
+// Bound by latency: rows that fit the CTA's registers (two 16-byte pieces a thread) are read once, together with their
+// weights.  Rows of 4096 with the residual, in a chain of launches: 2.6 -> 1.9 us at B = 1, 3.8 us at B = 256 as before.
 template <bool kAdd>
 __global__ void __launch_bounds__(1024)
 rms_norm_kernel(float* __restrict__ x, const float* __restrict__ residual, const float* __restrict__ weight,
                 int16_t* __restrict__ y, int n, float eps)
 {
-    __shared__ float scratch[33];
+    __shared__ float scratch[32];
     grid_launch_dependents();
-    grid_dependency_wait();
     const size_t off = (size_t)blockIdx.x * n;
-    float ss = 0.f;
     const bool vec = (n & 3) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(weight) |
                                        (kAdd ? reinterpret_cast<uintptr_t>(residual) : 0)) & 15) == 0 &&
                      (reinterpret_cast<uintptr_t>(y) & 7) == 0;
+    float4* x4 = reinterpret_cast<float4*>(x + off);
+    const float4* r4 = reinterpret_cast<const float4*>(residual + (kAdd ? off : 0));
+    const float4* w4 = reinterpret_cast<const float4*>(weight);
+    auto emit = [&](int i, const float4& v, const float4& w, float rms) {
+        const uint32_t lo = (uint16_t)float_to_bf16_rne(v.x * rms * w.x) | ((uint32_t)(uint16_t)float_to_bf16_rne(v.y * rms * w.y) << 16);
+        const uint32_t hi = (uint16_t)float_to_bf16_rne(v.z * rms * w.z) | ((uint32_t)(uint16_t)float_to_bf16_rne(v.w * rms * w.w) << 16);
+        reinterpret_cast<uint2*>(y + off)[i] = make_uint2(lo, hi);
+    };
+    float ss = 0.f;
+    grid_dependency_wait();
+    if (vec && n / 4 <= 2 * (int)blockDim.x) {
+        float4 v[2], w[2], r[2];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int i = threadIdx.x + j * blockDim.x;
+            if (i >= n / 4) continue;
+            v[j] = x4[i]; w[j] = w4[i];
+            if (kAdd) r[j] = r4[i];
+        }
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int i = threadIdx.x + j * blockDim.x;
+            if (i >= n / 4) continue;
+            if (kAdd) { v[j].x += r[j].x; v[j].y += r[j].y; v[j].z += r[j].z; v[j].w += r[j].w; x4[i] = v[j]; }
+            ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+        }
+        ss = block_sum(ss, scratch);
+        const float rms = rsqrtf(ss / (float)n + eps);
+#pragma unroll
+        for (int j = 0; j < 2; j++) { const int i = threadIdx.x + j * blockDim.x; if (i < n / 4) emit(i, v[j], w[j], rms); }
+        return;
+    }
     if (vec) {                                                    // 16-byte aligned rows: four elements per load
-        float4* x4 = reinterpret_cast<float4*>(x + off);
-        const float4* r4 = reinterpret_cast<const float4*>(residual + (kAdd ? off : 0));
         for (int i = threadIdx.x; i < n / 4; i += blockDim.x) {
             float4 v = x4[i];
             if (kAdd) { const float4 r = r4[i]; v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w; x4[i] = v; }
             ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
         }
-        ss = block_reduce<false>(ss, scratch);
+        ss = block_sum(ss, scratch);
         const float rms = rsqrtf(ss / (float)n + eps);
-        const float4* w4 = reinterpret_cast<const float4*>(weight);
-        for (int i = threadIdx.x; i < n / 4; i += blockDim.x) {
-            const float4 v = x4[i], w = w4[i];                    // a thread re-reads only what it wrote
-            const uint32_t lo = (uint16_t)float_to_bf16_rne(v.x * rms * w.x) | ((uint32_t)(uint16_t)float_to_bf16_rne(v.y * rms * w.y) << 16);
-            const uint32_t hi = (uint16_t)float_to_bf16_rne(v.z * rms * w.z) | ((uint32_t)(uint16_t)float_to_bf16_rne(v.w * rms * w.w) << 16);
-            reinterpret_cast<uint2*>(y + off)[i] = make_uint2(lo, hi);
-        }
+        for (int i = threadIdx.x; i < n / 4; i += blockDim.x) emit(i, x4[i], w4[i], rms);   // a thread re-reads only what it wrote
         return;
     }
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -119,7 +131,7 @@ rms_norm_kernel(float* __restrict__ x, const float* __restrict__ residual, const
         if (kAdd) { v += residual[off + i]; x[off + i] = v; }
         ss += v * v;
     }
-    ss = block_reduce<false>(ss, scratch);
+    ss = block_sum(ss, scratch);
     const float rms = rsqrtf(ss / (float)n + eps);
     for (int i = threadIdx.x; i < n; i += blockDim.x)
         y[off + i] = float_to_bf16_rne(x[off + i] * rms * weight[i]);    // a thread re-reads only what it wrote
@@ -162,9 +174,9 @@ add_kernel(float* __restrict__ y, const float* __restrict__ x, long long total)
 // RoPE on q and k (rotate-half form, engine/kernels.hip:174-215, 717-756) and
 // INT8 KV store with one scale per (position, kv head): scale = absmax/127,
 // value = clamp(rint(v * 127/absmax), -127, 127) (engine/kernels.hip:220-303,
-// 760-845).  One launch: CTA (h, seq) with h < n_head rotates q head h;
+// 760-845).  One launch: warp (h, seq) with h < n_head rotates q head h;
 // n_head <= h < n_head + n_head_kv rotates k head (written back, as the engine
-// does) and stores it; the last n_head_kv CTAs store v.  store == 0: rotation
+// does) and stores it; the last n_head_kv warps store v.  store == 0: rotation
 // only (launch_rope_batch); rope == 0: store only (launch_store_kv_batch).
 // ---------------------------------------------------------------------------
 struct RopeFreqs { float f[128]; };                              // head_dim <= 256
@@ -180,59 +192,61 @@ struct RopeKvParams {
     int rope, store;
 };
 
-__global__ void __launch_bounds__(256)
+constexpr int kRopeWarps = 4;
+
+// A warp per head, no shared memory: a lane owns elements d and d + half for d = lane, lane + 32, ... (at most four
+// pairs).  Bound by latency.  With a CTA of 128 threads and two block reductions per head (a third of the threads at
+// work) B = 256 took 13.1 us in a chain of launches (32 + 8 heads of 128), this way 8.0; B = 1 takes 2.3 us (2.0 before:
+// two sines a lane instead of one).  Five heads a warp, with the sines computed once: 9.4 us at B = 256.
+__global__ void __launch_bounds__(kRopeWarps * 32)
 rope_kv_kernel(const __grid_constant__ RopeKvParams P, const __grid_constant__ RopeFreqs F)
 {
-    __shared__ float scratch[33];
     grid_launch_dependents();
     grid_dependency_wait();
-    const int h = blockIdx.x, seq = blockIdx.y, d = threadIdx.x;
+    const int lane = threadIdx.x & 31, h = blockIdx.x * kRopeWarps + (threadIdx.x >> 5), seq = blockIdx.y;
     const int hd = P.head_dim, half = hd >> 1;
+    if (h >= P.n_head + P.n_head_kv * (P.store ? 2 : 1)) return;
     const int pos = P.positions ? P.positions[seq] : P.position;
-    if (h < P.n_head) {
-        if (P.rope && d < half) {
-            float* p = P.q + (size_t)seq * P.q_stride + (size_t)h * hd;
+    const bool is_q = h < P.n_head, is_v = h >= P.n_head + P.n_head_kv;
+    const int kvh = is_q ? h : h - P.n_head - (is_v ? P.n_head_kv : 0);
+    float* p = is_q ? P.q + (size_t)seq * P.q_stride + (size_t)h * hd
+                    : (is_v ? const_cast<float*>(P.v) : P.k) + (size_t)seq * P.k_stride + (size_t)kvh * hd;
+    float lo[4], hi[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int d = i * 32 + lane;
+        lo[i] = d < half ? p[d] : 0.f;
+        hi[i] = d < half ? p[d + half] : 0.f;
+    }
+    if (P.rope && !is_v) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int d = i * 32 + lane;
+            if (d >= half) break;
             float s, c;
             sincosf((float)pos * F.f[d], &s, &c);
-            const float x0 = p[d], x1 = p[d + half];
-            p[d] = x0 * c - x1 * s;
-            p[d + half] = x0 * s + x1 * c;
+            const float x0 = lo[i], x1 = hi[i];
+            lo[i] = x0 * c - x1 * s; hi[i] = x0 * s + x1 * c;
+            p[d] = lo[i]; p[d + half] = hi[i];
         }
-        return;
     }
-    const bool is_v = h >= P.n_head + P.n_head_kv;
-    const int kvh = h - P.n_head - (is_v ? P.n_head_kv : 0);
-    float val = 0.f;
-    if (!is_v) {
-        float* p = P.k + (size_t)seq * P.k_stride + (size_t)kvh * hd;
-        if (P.rope) {
-            float lo = 0.f, hi = 0.f;
-            if (d < half) {
-                float s, c;
-                sincosf((float)pos * F.f[d], &s, &c);
-                const float x0 = p[d], x1 = p[d + half];
-                lo = x0 * c - x1 * s; hi = x0 * s + x1 * c;
-                p[d] = lo; p[d + half] = hi;
-            }
-            // thread d needs element d: the upper half comes from thread d - half
-            __shared__ float rot[256];
-            if (d < half) { rot[d] = lo; rot[d + half] = hi; }
-            __syncthreads();
-            if (d < hd) val = rot[d];
-        } else if (d < hd) {
-            val = p[d];
-        }
-    } else if (d < hd) {
-        val = P.v[(size_t)seq * P.k_stride + (size_t)kvh * hd + d];
-    }
-    if (!P.store) return;
-    const float amax = block_reduce<true>(d < hd ? fabsf(val) : 0.f, scratch);
+    if (is_q || !P.store) return;
+    float amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) amax = fmaxf(amax, fmaxf(fabsf(lo[i]), fabsf(hi[i])));
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, off));
     const float inv = amax > 0.f ? 127.0f / amax : 0.f;
     const size_t kv_dim = (size_t)P.n_head_kv * hd;
     int8_t* dst = (is_v ? P.kv_v : P.kv_k) + (size_t)seq * P.kv_stride + (size_t)pos * kv_dim + (size_t)kvh * hd;
     float* sc = (is_v ? P.sc_v : P.sc_k) + (size_t)seq * (P.kv_stride / hd) + (size_t)pos * P.n_head_kv + kvh;
-    if (d < hd) dst[d] = (int8_t)(int)fminf(fmaxf(rintf(val * inv), -127.f), 127.f);
-    if (d == 0) *sc = amax / 127.0f;
+    auto quantise = [&](float v) { return (int8_t)(int)fminf(fmaxf(rintf(v * inv), -127.f), 127.f); };
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int d = i * 32 + lane;
+        if (d < half) { dst[d] = quantise(lo[i]); dst[d + half] = quantise(hi[i]); }
+    }
+    if (lane == 0) *sc = amax / 127.0f;
 }
 
 // ---------------------------------------------------------------------------
@@ -1002,14 +1016,11 @@ static int rope_kv_launch(RopeKvParams& P, float theta, int batch, void* stream,
         return fail(S12_ERR_UNSUPPORTED, "%s: head_dim must be even and <= 256, n_head_kv >= 1, batch >= 1", who);
     RopeFreqs F;
     rope_freqs(P.head_dim, theta, F);
-    const int threads = ((P.head_dim + 31) / 32) * 32;
-    const int heads = (P.rope ? P.n_head : 0);
-    // CTAs that would have nothing to do are not launched: q heads only when rotating, v heads only when storing
+    // heads that would have nothing to do get no warp: q heads only when rotating, v heads only when storing
     RopeKvParams Q = P;
-    if (!P.rope) { Q.n_head = 0; }
-    const int ctas = Q.n_head + P.n_head_kv + (P.store ? P.n_head_kv : 0);
-    (void)heads;
-    return launch(rope_kv_kernel, dim3(ctas, batch), dim3(threads), 0, stream, who, Q, F);
+    if (!P.rope) Q.n_head = 0;
+    const int heads = Q.n_head + P.n_head_kv * (P.store ? 2 : 1);
+    return launch(rope_kv_kernel, dim3((heads + kRopeWarps - 1) / kRopeWarps, batch), dim3(kRopeWarps * 32), 0, stream, who, Q, F);
 }
 
 // Launches attention_mma_kernel when it takes the shape (returns its status, 0 or negative), else returns 1.
