@@ -306,33 +306,34 @@ __device__ __forceinline__ void esc_advance(EscCursor& e, const GemmTensor& T)
 // (v[i] holds columns k0 + 2i and k0 + 2i + 1) and moves the cursor past k0 + 64.
 __device__ __forceinline__ void esc_apply(EscCursor& e, const GemmTensor& T, int k0, uint32_t (&v)[32])
 {
+    // The columns of the other groups, in a loop of their own: in one loop with the patch, some lane patches in nearly
+    // every round and all wait for it (expert block with 0.25 % escapes 647 -> 606 us).
+    while (e.c0 < k0) esc_advance(e, T);
     while (e.c0 < k0 + kTK) {
         const int idx = e.c0 - k0;
-        if (idx >= 0) {
-            const uint32_t keep = (idx & 1) ? 0x0000FFFFu : 0xFFFF0000u, ins = (idx & 1) ? (e.v0 << 16) : e.v0;
-            // One predicated (v & keep) | ins per register of the quarter that holds the entry, behind a branch per
-            // quarter (a warp rarely has more than one entry at a time).  Written as PTX so that the register array
-            // is not turned into an indexed local-memory array.  With all 32 registers tested for every entry, the
-            // escapes cost a tenth of a launch at B = 64 and 0.015 % escapes (28672 x 4096: 47.4 us, 42.0 without them,
-            // 45.9 this way), and a fifth of the time of 14336 x 4096 experts with 0.25 % (whole block 740 -> 653 us).
-            const int h = idx >> 1;
+        const uint32_t keep = (idx & 1) ? 0x0000FFFFu : 0xFFFF0000u, ins = (idx & 1) ? (e.v0 << 16) : e.v0;
+        // One predicated (v & keep) | ins per register of the quarter that holds the entry, behind a branch per
+        // quarter (a warp rarely has more than one entry at a time).  Written as PTX so that the register array
+        // is not turned into an indexed local-memory array.  With all 32 registers tested for every entry, the
+        // escapes cost a tenth of a launch at B = 64 and 0.015 % escapes (28672 x 4096: 47.4 us, 42.0 without them,
+        // 45.9 this way), and a fifth of the time of 14336 x 4096 experts with 0.25 % (whole block 740 -> 653 us).
+        const int h = idx >> 1;
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-                asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\t"
-                             "shr.s32 t, %8, 3;\n\tsetp.ne.s32 p, t, %11;\n\t@p bra ESC_SKIP%=;\n\tand.b32 t, %8, 7;\n\t"
-                             "setp.eq.s32 p, t, 0;\n\t@p lop3.b32 %0, %0, %9, %10, 0xEA;\n\t"
-                             "setp.eq.s32 p, t, 1;\n\t@p lop3.b32 %1, %1, %9, %10, 0xEA;\n\t"
-                             "setp.eq.s32 p, t, 2;\n\t@p lop3.b32 %2, %2, %9, %10, 0xEA;\n\t"
-                             "setp.eq.s32 p, t, 3;\n\t@p lop3.b32 %3, %3, %9, %10, 0xEA;\n\t"
-                             "setp.eq.s32 p, t, 4;\n\t@p lop3.b32 %4, %4, %9, %10, 0xEA;\n\t"
-                             "setp.eq.s32 p, t, 5;\n\t@p lop3.b32 %5, %5, %9, %10, 0xEA;\n\t"
-                             "setp.eq.s32 p, t, 6;\n\t@p lop3.b32 %6, %6, %9, %10, 0xEA;\n\t"
-                             "setp.eq.s32 p, t, 7;\n\t@p lop3.b32 %7, %7, %9, %10, 0xEA;\n\t"
-                             "ESC_SKIP%=:\n\t}"
-                             : "+r"(v[8 * q]), "+r"(v[8 * q + 1]), "+r"(v[8 * q + 2]), "+r"(v[8 * q + 3]), "+r"(v[8 * q + 4]),
-                               "+r"(v[8 * q + 5]), "+r"(v[8 * q + 6]), "+r"(v[8 * q + 7])
-                             : "r"(h), "r"(keep), "r"(ins), "r"(q));
-        }
+        for (int q = 0; q < 4; q++)
+            asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\t"
+                         "shr.s32 t, %8, 3;\n\tsetp.ne.s32 p, t, %11;\n\t@p bra ESC_SKIP%=;\n\tand.b32 t, %8, 7;\n\t"
+                         "setp.eq.s32 p, t, 0;\n\t@p lop3.b32 %0, %0, %9, %10, 0xEA;\n\t"
+                         "setp.eq.s32 p, t, 1;\n\t@p lop3.b32 %1, %1, %9, %10, 0xEA;\n\t"
+                         "setp.eq.s32 p, t, 2;\n\t@p lop3.b32 %2, %2, %9, %10, 0xEA;\n\t"
+                         "setp.eq.s32 p, t, 3;\n\t@p lop3.b32 %3, %3, %9, %10, 0xEA;\n\t"
+                         "setp.eq.s32 p, t, 4;\n\t@p lop3.b32 %4, %4, %9, %10, 0xEA;\n\t"
+                         "setp.eq.s32 p, t, 5;\n\t@p lop3.b32 %5, %5, %9, %10, 0xEA;\n\t"
+                         "setp.eq.s32 p, t, 6;\n\t@p lop3.b32 %6, %6, %9, %10, 0xEA;\n\t"
+                         "setp.eq.s32 p, t, 7;\n\t@p lop3.b32 %7, %7, %9, %10, 0xEA;\n\t"
+                         "ESC_SKIP%=:\n\t}"
+                         : "+r"(v[8 * q]), "+r"(v[8 * q + 1]), "+r"(v[8 * q + 2]), "+r"(v[8 * q + 3]), "+r"(v[8 * q + 4]),
+                           "+r"(v[8 * q + 5]), "+r"(v[8 * q + 6]), "+r"(v[8 * q + 7])
+                         : "r"(h), "r"(keep), "r"(ins), "r"(q));
         esc_advance(e, T);
     }
 }
