@@ -529,9 +529,15 @@ attention_kernel(const __grid_constant__ AttnParams P)
 // The kernel above needs ~60 clocks for them (an int8 -> float conversion per element on the quarter-rate pipe, a
 // multiply-add per element and query head, the shuffles of the dot products): 0.8 TB/s at 24 sequences of 2-4 k
 // positions, 195 us.  Here both products are mma.m16n8k16 with the cache as the B operand, one kv head's query heads in
-// the A rows, and nothing is rounded on the way: an int8 is exact in bf16, and a 32-bit q (or softmax weight times value
-// scale) is cut into three bf16 pieces of 8 significant bits, which are exact together.  With up to four query heads
-// the pieces sit in rows 0-3, 4-7 and 8-11 of one MMA; with eight, in rows 0-7 and 8-15 of one and rows 0-7 of a second.
+// the A rows.  The operands are exact: an int8 is exact in bf16, and a 32-bit q (or softmax weight times value scale) is
+// cut into three bf16 pieces of 8 significant bits, which are exact together.  With up to four query heads the pieces
+// sit in rows 0-3, 4-7 and 8-11 of one MMA; with eight, in rows 0-7 and 8-15 of one and rows 8-15 of a second.
+// The sums are 32-bit.  An MMA cuts off what does not fit its accumulator, which is a bias that grows with the number of
+// MMAs chained on it: so the low pieces never share a row with the high ones (their additions would cut the large sum
+// once more), and the weighted values of a chunk start from zero and are added to the sums rounded to nearest.  Outputs
+// that are not the bf16 value nearest to the 64-bit result, of 10^4, general kernel / chained accumulators / as here:
+// 56 sequences of 3.5-7 k positions 5.8 / 9.2 / 4.1, with eight query heads per kv head 4.8 / 19.9 / 3.4; 256 of 8-16
+// positions, one query head 1.24 / 1.51 / 1.05.  The times are the same (752 / 215 / 210 us, 14.3 / 12.7 / 12.3 us).
 // A warp walks chunks of 16 positions with a running maximum; cp.async keeps two or three chunks (8-12 KB) in flight per
 // warp, sixteen warps per SM (128 registers: q is read from shared memory again for every chunk; with q in registers
 // twelve warps were resident: 31 against 30 us on 256 x 192 positions, 51 against 53 on 24 x 4096).  The partial results
@@ -699,11 +705,11 @@ attention_mma_kernel(const __grid_constant__ AttnParams P)
     const uint2* q_row = pieces + head * kPieceRow + (kHD == 96 ? t4 * 2 : t4 * 4) + (kWide || g < 4 ? 0 : kHeads * kPieceRow);
     const float to_log2 = P.scale * 1.4426950408889634f;           // weights are powers of two of the scaled scores
 
-    float acc[kTiles][4];
+    float acc[kTiles][2];
 #pragma unroll
     for (int j = 0; j < kTiles; j++)
 #pragma unroll
-        for (int e = 0; e < 4; e++) acc[j][e] = 0.f;
+        for (int e = 0; e < 2; e++) acc[j][e] = 0.f;
     float m = -1e30f, l = 0.f;
 #pragma unroll 1
     for (int i = 0; i < n; i++) {
@@ -714,7 +720,7 @@ attention_mma_kernel(const __grid_constant__ AttnParams P)
         const uint8_t* V = K + kMmaPos * kHD;
         const float* sc = reinterpret_cast<const float*>(V + kMmaPos * kHD);
         const int t0 = first + i * stride + 2 * t4;                // this lane's positions: t0 + 8 u + {0, 1}
-        float w[2][2];
+        float dot[2][2], to_w[2][2];                               // a score is their product
         float mx = -1e30f;
         uint32_t kw[2][kSteps];
 #pragma unroll
@@ -746,7 +752,7 @@ attention_mma_kernel(const __grid_constant__ AttnParams P)
             for (int u = 0; u < 2; u++) {
                 const uint32_t b0 = s8_pair_to_bf16(kw[u][s]), b1 = s8_pair_to_bf16(kw[u][s] >> 8);
                 mma_bf16_16816(c[u], x0.x, x1.x, x0.y, x1.y, b0, b1);
-                if (kWide) mma_bf16_16816(c[u], x2.x, 0u, x2.y, 0u, b0, b1);
+                if (kWide) mma_bf16_16816(c[u], 0u, x2.x, 0u, x2.y, b0, b1);
             }
         }
 #pragma unroll
@@ -755,24 +761,24 @@ attention_mma_kernel(const __grid_constant__ AttnParams P)
             for (int e = 0; e < 2; e++) {
                 float x = c[u][e] + c[u][2 + e];
                 if (!kWide) x += __shfl_xor_sync(0xFFFFFFFFu, x, 16);
-                x *= sc[u * 8 + 2 * t4 + e] * to_log2;
-                w[u][e] = x;
-                if (t0 + u * 8 + e < t_hi) mx = fmaxf(mx, x);
+                dot[u][e] = x;
+                to_w[u][e] = sc[u * 8 + 2 * t4 + e] * to_log2;
+                if (t0 + u * 8 + e < t_hi) mx = fmaxf(mx, x * to_w[u][e]);
             }
         }
         mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 2));
-        // Weights are 2^(score - m) with m at least the maximum so far; it is set six above a new maximum, so that the
-        // sums are rarely rescaled.
+        // Weights are 2^(score - m), the difference rounded once.  m is at least the maximum so far: two above a new one,
+        // so that the sums are rarely rescaled, and a whole number, so that rescaling is exact.
         if (__any_sync(0xFFFFFFFFu, mx > m)) {
-            const float mn = mx > m ? mx + 6.f : m, f = exp2_approx(m - mn);
+            const float mn = mx > m ? ceilf(mx) + 2.f : m, f = exp2_approx(m - mn);
             m = mn;
             if (i > 0) {
                 l *= f;
 #pragma unroll
                 for (int j = 0; j < kTiles; j++)
 #pragma unroll
-                    for (int e = 0; e < 4; e++) acc[j][e] *= f;
+                    for (int e = 0; e < 2; e++) acc[j][e] *= f;
             }
         }
         uint32_t ap[4], apl[2];
@@ -782,7 +788,7 @@ attention_mma_kernel(const __grid_constant__ AttnParams P)
 #pragma unroll
             for (int e = 0; e < 2; e++) {
                 const bool live = t0 + u * 8 + e < t_hi;
-                const float p = live ? exp2_approx(w[u][e] - m) : 0.f;
+                const float p = live ? exp2_approx(fmaf(dot[u][e], to_w[u][e], -m)) : 0.f;
                 l += p;
                 split_product_bf16x3(live ? p * sc[kMmaPos + u * 8 + 2 * t4 + e] : 0.f, hi[e], mid[e], lo[e]);
             }
@@ -819,9 +825,10 @@ attention_mma_kernel(const __grid_constant__ AttnParams P)
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
                     const uint32_t b0 = s8_pair_to_bf16(e ? x0 >> 8 : x0), b1 = s8_pair_to_bf16(e ? x1 >> 8 : x1);
-                    float (&c)[4] = acc[4 * b + 2 * h + e];
+                    float c[4] = {0.f, 0.f, 0.f, 0.f}, (&sum)[2] = acc[4 * b + 2 * h + e];
                     mma_bf16_16816(c, ap[0], ap[1], ap[2], ap[3], b0, b1);
-                    if (kWide) mma_bf16_16816(c, apl[0], 0u, apl[1], 0u, b0, b1);
+                    if (kWide) mma_bf16_16816(c, 0u, apl[0], 0u, apl[1], b0, b1);
+                    sum[0] += c[0] + c[2]; sum[1] += c[1] + c[3];
                 }
             }
     }
@@ -838,7 +845,7 @@ attention_mma_kernel(const __grid_constant__ AttnParams P)
             float x[4];
 #pragma unroll
             for (int d = 0; d < 4; d++) {
-                x[d] = acc[j + d][e] + acc[j + d][2 + e];
+                x[d] = acc[j + d][e];
                 if (!kWide) x[d] += __shfl_xor_sync(0xFFFFFFFFu, x[d], 16);
             }
             if (owner) *reinterpret_cast<float4*>(mine + head * mma_acc_row(kHD) + (2 * t4 + e) * mma_acc_col(kHD) + j) = make_float4(x[0], x[1], x[2], x[3]);
