@@ -112,3 +112,26 @@ def test_as_near_to_64_bits_as_the_general_kernel(n_kv, gqa, hd, B, T):
             for i in range(2):
                 wrong[i] += int((outs[i][b] != want).sum())
     assert wrong[0] <= wrong[1] + 4.0 * (wrong[0] + wrong[1]) ** 0.5, wrong
+
+
+@pytest.mark.parametrize("hd,off", [(128, 0), (64, 0), (128, 4), (80, 0)])
+@pytest.mark.parametrize("bound", [1, 17, 101, 1003])
+def test_positions_past_the_bound_read_nothing_past_it(hd, off, bound):
+    """Device positions at and past the caller's bound give the result at the bound, in both kernels (a cache 4 bytes off
+    a 16-byte boundary and a head size of 80 take the general one).  The cache goes on past the bound, with values that would show."""
+    import torch
+    from turbo_lossless_b200 import Split12Engine
+    eng = Split12Engine()
+    g = torch.Generator(device="cuda").manual_seed(bound)
+    n_kv, B, room = 2, 3, bound + 64
+    kv = [torch.randint(-127, 128, (B * room * n_kv * hd + 16,), dtype=torch.int8, device="cuda", generator=g) for _ in range(2)]
+    q = torch.randn(B, 8 * hd, device="cuda", generator=g)
+    sk, sv = (0.01 + 0.02 * torch.rand(B, room, n_kv, device="cuda", generator=g) for _ in range(2))
+    sv[:, bound:] = 1e9
+    outs = []
+    for at in (bound - 1, bound, bound + 40):
+        out = torch.zeros(B, 8 * hd, dtype=torch.int16, device="cuda")
+        pos = torch.full((B,), at, dtype=torch.int32, device="cuda")
+        eng.attention_all_heads_batch(q, kv[0][off:], kv[1][off:], sk, sv, out, pos, 8, n_kv, hd, bound, hd ** -0.5, B, room * n_kv * hd)
+        outs.append(out)
+    assert outs[0].any() and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])

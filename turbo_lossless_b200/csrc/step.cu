@@ -276,7 +276,7 @@ struct AttnParams {
     float scale;
     int score_stride;           // floats between the score rows of two query heads in shared memory
     int nsplit;                 // CTAs (= cluster size) that share the positions of one (kv head, sequence)
-    int t_limit;                // positions a launch may read, whatever `positions` holds
+    int t_limit;                // the caller's bound: positions a launch may read, whatever `positions` holds
     int stages;                 // attention_mma_kernel: chunks of a warp's ring in shared memory
 };
 
@@ -319,7 +319,7 @@ attention_kernel(const __grid_constant__ AttnParams P)
     const int kvh = blockIdx.x, seq = blockIdx.y, split = blockIdx.z, nsplit = P.nsplit;
     const int hd = P.head_dim;
     const int Tw = P.positions ? P.positions[seq] + 1 : P.seq_len;
-    const int T = Tw < P.t_limit ? Tw : P.t_limit;                 // never past what this launch was sized for
+    const int T = Tw < P.t_limit ? Tw : P.t_limit;                 // never past the caller's bound
     const int per = (T + nsplit - 1) / nsplit;
     const int t_lo = split * per, t_hi = t_lo + per < T ? t_lo + per : T;       // this CTA's positions
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1095,7 +1095,7 @@ static int attention_launch(AttnParams& P, int max_len, int batch, void* stream,
     P.score_stride = (per + 3) & ~3;
     const size_t smem = smem_for(nsplit);
     if (smem > 200 * 1024) return fail(S12_ERR_TOO_LARGE, "%s: seq_len %d needs more shared memory than one CTA has", who, max_len);
-    P.t_limit = P.score_stride * nsplit;
+    P.t_limit = max_len;
     const int mma = attention_mma_launch(P, gqa, max_len, batch, stream, who);
     if (mma <= 0) return mma;
     typedef void (*Kern)(const AttnParams);
