@@ -106,3 +106,23 @@ def test_given_window_over_every_value(O, base_exp):
     assert cw.num_patches == len(cols) and np.array_equal(cw.patch_cols.cpu().numpy(), cols)
     assert np.array_equal(cw.row_offsets.cpu().numpy(), np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=256))]))
     assert np.array_equal(cw.patch_correct.cpu().numpy().view(np.uint16), w[rows, cols])
+
+
+def test_rows_within_a_scan_round_of_the_largest_int():
+    """As many rows as a 32-bit count holds, less than the scan's 8192 rows from its end (24 GB of tensors)."""
+    from turbo_lossless_b200 import capi
+    from turbo_lossless_b200.capi import check
+    M, K = 2 ** 31 - 6000, 2
+    if torch.cuda.mem_get_info()[0] < 40e9:
+        pytest.skip("needs 24 GB of device memory")
+    w = torch.full((M * K,), 0x3F80, dtype=torch.int16, device="cuda")            # 1.0: exponent 127
+    rows = torch.tensor([0, 1023, 8191, 8192, 5 * 10 ** 8, M - 8192, M - 2, M - 1], device="cuda")
+    w[rows * K + 1] = 0
+    sm, gr = (torch.empty(M * K // n, dtype=torch.uint8, device="cuda") for n in (1, 2))
+    row_off = torch.empty(M + 1, dtype=torch.int32, device="cuda")
+    check(capi.load().s12_pack_async(w.data_ptr(), M, K, 120, sm.data_ptr(), gr.data_ptr(), row_off.data_ptr(), None))
+    for a in range(0, M + 1, 1 << 28):
+        at = torch.arange(a, min(a + (1 << 28), M + 1), device="cuda")
+        assert torch.equal(row_off[a:a + (1 << 28)], torch.searchsorted(rows, at, out_int32=True))   # escapes in the rows before
+    del w, sm, gr, row_off, at
+    torch.cuda.empty_cache()                                                     # later tests watch the driver's allocations

@@ -191,11 +191,11 @@ scan_kernel(int32_t* __restrict__ row_off, int M, int* __restrict__ total)
     __shared__ int piece[kScanRows * 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int carry = 0;
-    for (int base = 1; base <= M; base += kScanRows * 1024) {
+    for (int64_t base = 1; base <= M; base += kScanRows * 1024) {   // 64 bits: M may lie within a round of 2^31
         int v[kScanRows];
 #pragma unroll
         for (int j = 0; j < kScanRows; j++) {
-            const int64_t i = (int64_t)base + j * 1024 + threadIdx.x;
+            const int64_t i = base + j * 1024 + threadIdx.x;
             v[j] = i <= M ? row_off[i] : 0;
         }
 #pragma unroll
@@ -226,7 +226,7 @@ scan_kernel(int32_t* __restrict__ row_off, int M, int* __restrict__ total)
         int last = 0;
 #pragma unroll
         for (int j = 0; j < kScanRows; j++) {
-            const int64_t i = (int64_t)base + j * 1024 + threadIdx.x;
+            const int64_t i = base + j * 1024 + threadIdx.x;
             v[j] += piece[j * 32 + warp] + carry;
             if (i <= M) row_off[i] = v[j];
             last = v[j];
