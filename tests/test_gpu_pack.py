@@ -65,10 +65,10 @@ def test_pack_under_dependent_launch(O, golden):
 
 
 @pytest.mark.parametrize("M,K,frac", [(1, 2, 1.0), (5, 6, 0.5), (3, 8, 0.3), (7, 24, 0.2), (2, 1032, 0.1), (3, 4104, 1e-2), (1, 16384, 0.9),
-                                      (9, 2056, 0.33), (40, 264, 0.34), (40, 248, 0.34), (1023, 16, 0.2), (8191, 8, 0.1), (8192, 34, 0.05), (8193, 16, 0.1), (20000, 40, 0.02)])
+                                      (9, 2056, 0.33), (40, 264, 0.34), (40, 248, 0.34), (1023, 16, 0.2), (1025, 16, 0.2), (2049, 8, 0.2), (4097, 6, 0.1), (8191, 8, 0.1), (8192, 34, 0.05), (8193, 16, 0.1), (20000, 40, 0.02)])
 @pytest.mark.parametrize("offset", [0, 1, 8])
 def test_edges_of_the_passes(O, M, K, frac, offset):
-    """Rows around the scan's 8192, columns around the fill's 256 and 1024, values off a 16-byte boundary (offset
+    """Rows around the scan's 1024 to 8192, columns around the fill's 256 and 1024, values off a 16-byte boundary (offset
     elements into a buffer): one call, and the separate passes on the same values."""
     from turbo_lossless_b200 import CompressedWeight, capi
     from turbo_lossless_b200.capi import check

@@ -181,25 +181,26 @@ pack2_kernel(const uint16_t* __restrict__ w, int64_t num_pairs, int K, const Bas
 }
 
 // In-place inclusive scan of row_off[1..M] (row_off[0] == 0), one CTA; the sum also goes to *total when it is given.
-// A round takes 8192 rows: each thread loads eight, 1024 apart (coalesced, and one latency for all), the warps scan
-// their 8 x 32 pieces, one warp scans the 256 pieces' sums.
-constexpr int kScanRows = 8;
+// A round takes 1024 x kRows rows: each thread loads kRows, 1024 apart (coalesced, and one latency for all), the warps scan
+// their kRows x 32 pieces, one warp scans the pieces' sums.  kRows is the smallest with which one round will do, up to
+// eight: with eight for all, the scan of up to 1024 rows took 1-2 us longer (pack + scan of 512 x 512 6.3 -> 8.2 us).
+template <int kRows>
 __global__ void __launch_bounds__(1024)
 scan_kernel(int32_t* __restrict__ row_off, int M, int* __restrict__ total)
 {
     grid_dependency_wait();                    // the per-row counts come from the pack kernel before
-    __shared__ int piece[kScanRows * 32];
+    __shared__ int piece[kRows * 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int carry = 0;
-    for (int64_t base = 1; base <= M; base += kScanRows * 1024) {   // 64 bits: M may lie within a round of 2^31
-        int v[kScanRows];
+    for (int64_t base = 1; base <= M; base += kRows * 1024) {   // 64 bits: M may lie within a round of 2^31
+        int v[kRows];
 #pragma unroll
-        for (int j = 0; j < kScanRows; j++) {
+        for (int j = 0; j < kRows; j++) {
             const int64_t i = base + j * 1024 + threadIdx.x;
             v[j] = i <= M ? row_off[i] : 0;
         }
 #pragma unroll
-        for (int j = 0; j < kScanRows; j++) {
+        for (int j = 0; j < kRows; j++) {
 #pragma unroll
             for (int off = 1; off < 32; off <<= 1) {
                 const int t = __shfl_up_sync(0xFFFFFFFFu, v[j], off);
@@ -208,10 +209,10 @@ scan_kernel(int32_t* __restrict__ row_off, int M, int* __restrict__ total)
             if (lane == 31) piece[j * 32 + warp] = v[j];
         }
         __syncthreads();
-        if (warp == 0) {                                         // exclusive scan of the 256 sums, eight a lane
-            int s[8], sum = 0;
+        if (warp == 0) {                                         // exclusive scan of the sums, kRows a lane
+            int s[kRows], sum = 0;
 #pragma unroll
-            for (int k = 0; k < 8; k++) { s[k] = sum; sum += piece[lane * 8 + k]; }
+            for (int k = 0; k < kRows; k++) { s[k] = sum; sum += piece[lane * kRows + k]; }
             int before = sum;
 #pragma unroll
             for (int off = 1; off < 32; off <<= 1) {
@@ -220,12 +221,12 @@ scan_kernel(int32_t* __restrict__ row_off, int M, int* __restrict__ total)
             }
             before -= sum;
 #pragma unroll
-            for (int k = 0; k < 8; k++) piece[lane * 8 + k] = before + s[k];
+            for (int k = 0; k < kRows; k++) piece[lane * kRows + k] = before + s[k];
         }
         __syncthreads();
         int last = 0;
 #pragma unroll
-        for (int j = 0; j < kScanRows; j++) {
+        for (int j = 0; j < kRows; j++) {
             const int64_t i = base + j * 1024 + threadIdx.x;
             v[j] += piece[j * 32 + warp] + carry;
             if (i <= M) row_off[i] = v[j];
@@ -381,7 +382,8 @@ static int pack_launch(const void* bf16, int M, int K, const BaseExp& be, void* 
     const int rc = launch(vec ? pack16_kernel : pack2_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, who,
                           (const uint16_t*)bf16, items, K, be, (uint8_t*)sm, (uint8_t*)gr, (int32_t*)row_off);
     if (rc) return rc;
-    return launch(scan_kernel, dim3(1), dim3(1024), 0, stream, who, (int32_t*)row_off, M, total);
+    return launch(M <= 1024 ? scan_kernel<1> : M <= 2048 ? scan_kernel<2> : M <= 4096 ? scan_kernel<4> : scan_kernel<8>, dim3(1), dim3(1024), 0,
+                  stream, who, (int32_t*)row_off, M, total);
 }
 
 static int fill_launch(const void* bf16, const void* gr, int M, int K, int base_exp, const void* row_off, void* cols, void* correct,
