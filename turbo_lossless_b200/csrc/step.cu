@@ -189,64 +189,126 @@ struct RopeKvParams {
     int head_dim, n_head, n_head_kv;
     int q_stride, k_stride;     // floats between sequences in q and k/v
     long long kv_stride;        // int8 elements between the sequences' caches (0: one shared cache)
-    int rope, store;
+    int store;
+    int cta_slots;              // groups of warps of a CTA, each with heads of its own
 };
 
 constexpr int kRopeWarps = 4;
+__host__ __device__ constexpr int rope_head_warps(int head_dim) { return (head_dim / 2 + 31) / 32; }
 
-// A warp per head, no shared memory: a lane owns elements d and d + half for d = lane, lane + 32, ... (at most four
-// pairs).  Bound by latency.  With a CTA of 128 threads and two block reductions per head (a third of the threads at
-// work) B = 256 took 13.1 us in a chain of launches (32 + 8 heads of 128), this way 8.0; B = 1 takes 2.3 us (2.0 before:
-// two sines a lane instead of one).  Five heads a warp, with the sines computed once: 9.4 us at B = 256.
+__device__ __forceinline__ int8_t quantise(float v, float inv) { return (int8_t)(int)fminf(fmaxf(rintf(v * inv), -127.f), 127.f); }
+// where a kv head of this sequence's position lies in the caches
+struct KvSlot { int8_t* dst; float* scale; };
+__device__ __forceinline__ KvSlot kv_slot(const RopeKvParams& P, int seq, int pos, int kvh, bool is_v)
+{
+    return {(is_v ? P.kv_v : P.kv_k) + (size_t)seq * P.kv_stride + ((size_t)pos * P.n_head_kv + kvh) * P.head_dim,
+            (is_v ? P.sc_v : P.sc_k) + (size_t)seq * (P.kv_stride / P.head_dim) + (size_t)pos * P.n_head_kv + kvh};
+}
+
+// The store alone: a warp per head, no shared memory; a lane owns elements d and d + half for d = lane, lane + 32, ...
+// Bound by latency.  32 kv heads of 128 at B = 256: 5.4 us (a thread per pair, as below: 8.6); 8 at B = 1: 1.3 us.
 __global__ void __launch_bounds__(kRopeWarps * 32)
-rope_kv_kernel(const __grid_constant__ RopeKvParams P, const __grid_constant__ RopeFreqs F)
+store_kv_kernel(const __grid_constant__ RopeKvParams P)
 {
     grid_launch_dependents();
-    grid_dependency_wait();
     const int lane = threadIdx.x & 31, h = blockIdx.x * kRopeWarps + (threadIdx.x >> 5), seq = blockIdx.y;
     const int hd = P.head_dim, half = hd >> 1;
-    if (h >= P.n_head + P.n_head_kv * (P.store ? 2 : 1)) return;
+    if (h >= 2 * P.n_head_kv) return;
+    const bool is_v = h >= P.n_head_kv;
+    const int kvh = h - (is_v ? P.n_head_kv : 0);
+    const float* p = (is_v ? P.v : P.k) + (size_t)seq * P.k_stride + (size_t)kvh * hd;
+    grid_dependency_wait();
     const int pos = P.positions ? P.positions[seq] : P.position;
-    const bool is_q = h < P.n_head, is_v = h >= P.n_head + P.n_head_kv;
-    const int kvh = is_q ? h : h - P.n_head - (is_v ? P.n_head_kv : 0);
-    float* p = is_q ? P.q + (size_t)seq * P.q_stride + (size_t)h * hd
-                    : (is_v ? const_cast<float*>(P.v) : P.k) + (size_t)seq * P.k_stride + (size_t)kvh * hd;
-    float lo[4], hi[4];
+    float lo[4], hi[4], amax = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int d = i * 32 + lane;
         lo[i] = d < half ? p[d] : 0.f;
         hi[i] = d < half ? p[d + half] : 0.f;
     }
-    if (P.rope && !is_v) {
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int d = i * 32 + lane;
-            if (d >= half) break;
-            float s, c;
-            sincosf((float)pos * F.f[d], &s, &c);
-            const float x0 = lo[i], x1 = hi[i];
-            lo[i] = x0 * c - x1 * s; hi[i] = x0 * s + x1 * c;
-            p[d] = lo[i]; p[d + half] = hi[i];
-        }
-    }
-    if (is_q || !P.store) return;
-    float amax = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; i++) amax = fmaxf(amax, fmaxf(fabsf(lo[i]), fabsf(hi[i])));
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, off));
     const float inv = amax > 0.f ? 127.0f / amax : 0.f;
-    const size_t kv_dim = (size_t)P.n_head_kv * hd;
-    int8_t* dst = (is_v ? P.kv_v : P.kv_k) + (size_t)seq * P.kv_stride + (size_t)pos * kv_dim + (size_t)kvh * hd;
-    float* sc = (is_v ? P.sc_v : P.sc_k) + (size_t)seq * (P.kv_stride / hd) + (size_t)pos * P.n_head_kv + kvh;
-    auto quantise = [&](float v) { return (int8_t)(int)fminf(fmaxf(rintf(v * inv), -127.f), 127.f); };
+    const KvSlot at = kv_slot(P, seq, pos, kvh, is_v);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int d = i * 32 + lane;
-        if (d < half) { dst[d] = quantise(lo[i]); dst[d + half] = quantise(hi[i]); }
+        if (d < half) { at.dst[d] = quantise(lo[i], inv); at.dst[d + half] = quantise(hi[i], inv); }
     }
-    if (lane == 0) *sc = amax / 127.0f;
+    if (lane == 0) *at.scale = amax / 127.0f;
+}
+
+// A thread owns elements d and d + half of kHeads neighbouring heads, whose angles are the same, and runs sincosf once; a
+// head lies over ceil(half / 32) neighbouring warps of a CTA.  Bound by latency: the addresses are there before the wait
+// for the launch before.  In a chain of launches, 32 + 8 heads of 128, us at B = 1 / 64 / 256: a CTA per head with two
+// block reductions 2.0 / 4.4 / 13.1; a warp per head, two sines a lane one after the other, 2.3 / 4.2 / 8.1; this way with
+// one head a thread 1.75 / 3.8 / 8.8, with two 1.95 / 2.9 / 6.0.
+template <int kHeads>
+__global__ void __launch_bounds__(kRopeWarps * 32)
+rope_kv_kernel(const __grid_constant__ RopeKvParams P, const __grid_constant__ RopeFreqs F)
+{
+    __shared__ float top[kHeads][kRopeWarps];
+    grid_launch_dependents();
+    const int hd = P.head_dim, half = hd >> 1, wph = rope_head_warps(hd), slots = P.cta_slots;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, seq = blockIdx.y;
+    const int slot = slots == 4 ? warp : slots == 2 ? warp >> 1 : 0, d = (warp - slot * wph) * 32 + lane;
+    const int h0 = (blockIdx.x * slots + slot) * kHeads, first_v = P.n_head + P.n_head_kv, end = first_v + (P.store ? P.n_head_kv : 0);
+    float* p[kHeads];
+    bool live[kHeads];
+#pragma unroll
+    for (int j = 0; j < kHeads; j++) {
+        const int h = h0 + j;
+        live[j] = d < half && h < end;
+        p[j] = (h < P.n_head ? P.q + (size_t)seq * P.q_stride + (size_t)h * hd
+                             : (h < first_v ? P.k + (size_t)(h - P.n_head) * hd : const_cast<float*>(P.v) + (size_t)(h - first_v) * hd) + (size_t)seq * P.k_stride) + d;
+    }
+    grid_dependency_wait();
+    const int pos = P.positions ? P.positions[seq] : P.position;
+    float lo[kHeads], hi[kHeads];
+#pragma unroll
+    for (int j = 0; j < kHeads; j++) {
+        lo[j] = live[j] ? p[j][0] : 0.f;
+        hi[j] = live[j] ? p[j][half] : 0.f;
+    }
+    if (d < half && h0 < first_v) {
+        float s, c;
+        sincosf((float)pos * F.f[d], &s, &c);
+#pragma unroll
+        for (int j = 0; j < kHeads; j++) {
+            if (h0 + j >= first_v) break;
+            const float x0 = lo[j], x1 = hi[j];
+            lo[j] = x0 * c - x1 * s; hi[j] = x0 * s + x1 * c;
+            p[j][0] = lo[j]; p[j][half] = hi[j];
+        }
+    }
+    if (!P.store || (int)(blockIdx.x + 1) * slots * kHeads <= P.n_head) return;   // the whole CTA
+    float amax[kHeads];
+#pragma unroll
+    for (int j = 0; j < kHeads; j++) {
+        amax[j] = fmaxf(fabsf(lo[j]), fabsf(hi[j]));
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) amax[j] = fmaxf(amax[j], __shfl_xor_sync(0xFFFFFFFFu, amax[j], off));
+        if (lane == 0) top[j][warp] = amax[j];
+    }
+    if (wph > 1) {
+        __syncthreads();
+        for (int i = 0; i < wph; i++)
+#pragma unroll
+            for (int j = 0; j < kHeads; j++) amax[j] = fmaxf(amax[j], top[j][slot * wph + i]);
+    }
+#pragma unroll
+    for (int j = 0; j < kHeads; j++) {
+        const int h = h0 + j;
+        if (d >= half || h < P.n_head || h >= end) continue;
+        const bool is_v = h >= first_v;
+        const float inv = amax[j] > 0.f ? 127.0f / amax[j] : 0.f;
+        const KvSlot at = kv_slot(P, seq, pos, h - (is_v ? first_v : P.n_head), is_v);
+        at.dst[d] = quantise(lo[j], inv);
+        at.dst[d + half] = quantise(hi[j], inv);
+        if (d == 0) *at.scale = amax[j] / 127.0f;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1037,17 +1099,20 @@ static void rope_freqs(int head_dim, float theta, RopeFreqs& F)
     F = cached;
 }
 
-static int rope_kv_launch(RopeKvParams& P, float theta, int batch, void* stream, const char* who)
+static int rope_kv_launch(RopeKvParams P, bool rope, float theta, int batch, void* stream, const char* who)
 {
     if (P.head_dim < 2 || P.head_dim > 256 || (P.head_dim & 1) || P.n_head < 0 || P.n_head_kv < 1 || batch < 1)
         return fail(S12_ERR_UNSUPPORTED, "%s: head_dim must be even and <= 256, n_head_kv >= 1, batch >= 1", who);
+    if (!rope) return launch(store_kv_kernel, dim3((2 * P.n_head_kv + kRopeWarps - 1) / kRopeWarps, batch), dim3(kRopeWarps * 32), 0, stream, who, P);
     RopeFreqs F;
     rope_freqs(P.head_dim, theta, F);
-    // heads that would have nothing to do get no warp: q heads only when rotating, v heads only when storing
-    RopeKvParams Q = P;
-    if (!P.rope) Q.n_head = 0;
-    const int heads = Q.n_head + P.n_head_kv * (P.store ? 2 : 1);
-    return launch(rope_kv_kernel, dim3((heads + kRopeWarps - 1) / kRopeWarps, batch), dim3(kRopeWarps * 32), 0, stream, who, Q, F);
+    const int wph = rope_head_warps(P.head_dim), heads = P.n_head + P.n_head_kv * (P.store ? 2 : 1);
+    P.cta_slots = kRopeWarps / wph;
+    const int ctas = (heads + P.cta_slots - 1) / P.cta_slots;
+    // two heads a thread from three CTAs per SM on: 64 + 8 heads at B = 8 (320 CTAs) 2.2 us either way, at B = 16 3.0 -> 2.4
+    const int two = (long long)ctas * batch > 3ll * sm_count() ? 2 : 1;
+    return launch(two == 2 ? rope_kv_kernel<2> : rope_kv_kernel<1>, dim3((ctas + two - 1) / two, batch), dim3(P.cta_slots * wph * 32), 0, stream,
+                  who, P, F);
 }
 
 // Launches attention_mma_kernel when it takes the shape (returns its status, 0 or negative), else returns 1.
@@ -1210,8 +1275,8 @@ int launch_rope_store_kv(float* q, float* k, const float* v, int8_t* kv_k, int8_
     RopeKvParams P = {};
     P.q = q; P.k = k; P.v = v; P.kv_k = kv_k; P.kv_v = kv_v; P.sc_k = kv_scale_k; P.sc_v = kv_scale_v;
     P.position = position; P.head_dim = head_dim; P.n_head = n_head; P.n_head_kv = n_head_kv;
-    P.q_stride = n_head * head_dim; P.k_stride = n_head_kv * head_dim; P.rope = 1; P.store = 1;
-    return rope_kv_launch(P, theta, 1, stream, "launch_rope_store_kv");
+    P.q_stride = n_head * head_dim; P.k_stride = n_head_kv * head_dim; P.store = 1;
+    return rope_kv_launch(P, true, theta, 1, stream, "launch_rope_store_kv");
 }
 int launch_rope_batch(float* q, float* k, const int* positions, int head_dim, int n_head, int n_head_kv, int q_stride,
                       int k_stride, float theta, int batch_size, void* stream)
@@ -1219,8 +1284,8 @@ int launch_rope_batch(float* q, float* k, const int* positions, int head_dim, in
     if (!q || !k || !positions) return fail(S12_ERR_BAD_ARG, "launch_rope_batch: null argument");
     RopeKvParams P = {};
     P.q = q; P.k = k; P.positions = positions; P.head_dim = head_dim; P.n_head = n_head; P.n_head_kv = n_head_kv;
-    P.q_stride = q_stride; P.k_stride = k_stride; P.rope = 1; P.store = 0;
-    return rope_kv_launch(P, theta, batch_size, stream, "launch_rope_batch");
+    P.q_stride = q_stride; P.k_stride = k_stride; P.store = 0;
+    return rope_kv_launch(P, true, theta, batch_size, stream, "launch_rope_batch");
 }
 // The engine's batched store writes every sequence into ONE cache at its position
 // (engine/kernels.hip:784-788); s12_store_kv_batch below adds the per-sequence stride.
@@ -1231,8 +1296,8 @@ int s12_store_kv_batch(const float* k, const float* v, int8_t* kv_k, int8_t* kv_
     RopeKvParams P = {};
     P.k = const_cast<float*>(k); P.v = v; P.kv_k = kv_k; P.kv_v = kv_v; P.sc_k = kv_scale_k; P.sc_v = kv_scale_v;
     P.positions = positions; P.head_dim = head_dim; P.n_head = 0; P.n_head_kv = n_head_kv;
-    P.k_stride = n_head_kv * head_dim; P.kv_stride = kv_stride; P.rope = 0; P.store = 1;
-    return rope_kv_launch(P, 10000.0f, batch_size, stream, "store_kv_batch");
+    P.k_stride = n_head_kv * head_dim; P.kv_stride = kv_stride; P.store = 1;
+    return rope_kv_launch(P, false, 0.f, batch_size, stream, "store_kv_batch");
 }
 // launch_rope_batch and s12_store_kv_batch as one launch.
 int s12_rope_store_kv_batch(float* q, float* k, const float* v, int8_t* kv_k, int8_t* kv_v, float* kv_scale_k, float* kv_scale_v,
@@ -1244,8 +1309,8 @@ int s12_rope_store_kv_batch(float* q, float* k, const float* v, int8_t* kv_k, in
     RopeKvParams P = {};
     P.q = q; P.k = k; P.v = v; P.kv_k = kv_k; P.kv_v = kv_v; P.sc_k = kv_scale_k; P.sc_v = kv_scale_v;
     P.positions = positions; P.head_dim = head_dim; P.n_head = n_head; P.n_head_kv = n_head_kv;
-    P.q_stride = n_head * head_dim; P.k_stride = n_head_kv * head_dim; P.kv_stride = kv_stride; P.rope = 1; P.store = 1;
-    return rope_kv_launch(P, theta, batch_size, stream, "s12_rope_store_kv_batch");
+    P.q_stride = n_head * head_dim; P.k_stride = n_head_kv * head_dim; P.kv_stride = kv_stride; P.store = 1;
+    return rope_kv_launch(P, true, theta, batch_size, stream, "s12_rope_store_kv_batch");
 }
 int launch_store_kv_batch(const float* k, const float* v, int8_t* kv_k, int8_t* kv_v, float* kv_scale_k, float* kv_scale_v,
                           const int* positions, int kv_dim, int max_seq, int n_head_kv, int head_dim, int batch_size, void* stream)
