@@ -73,9 +73,8 @@ embed_kernel(const int16_t* __restrict__ table, const int* __restrict__ tokens, 
 // Bound by latency: rows that fit the CTA's registers (two 16-byte pieces a thread) are read once, together with their
 // weights.  Rows of 4096 with the residual, in a chain of launches: 2.6 -> 1.9 us at B = 1, 3.8 us at B = 256 as before.
 template <bool kAdd>
-__global__ void __launch_bounds__(1024)
-rms_norm_kernel(float* __restrict__ x, const float* __restrict__ residual, const float* __restrict__ weight,
-                int16_t* __restrict__ y, int n, float eps)
+__device__ __forceinline__ void rms_norm_row(float* __restrict__ x, const float* __restrict__ residual, const float* __restrict__ weight,
+                                             int16_t* __restrict__ y, int n, float eps)
 {
     __shared__ float scratch[32];
     grid_launch_dependents();
@@ -135,6 +134,22 @@ rms_norm_kernel(float* __restrict__ x, const float* __restrict__ residual, const
     const float rms = rsqrtf(ss / (float)n + eps);
     for (int i = threadIdx.x; i < n; i += blockDim.x)
         y[off + i] = float_to_bf16_rne(x[off + i] * rms * weight[i]);    // a thread re-reads only what it wrote
+}
+template <bool kAdd>
+__global__ void __launch_bounds__(1024)
+rms_norm_kernel(float* __restrict__ x, const float* __restrict__ residual, const float* __restrict__ weight,
+                int16_t* __restrict__ y, int n, float eps)
+{
+    rms_norm_row<kAdd>(x, residual, weight, y, n, eps);
+}
+// With the residual a thread takes 48 registers, and an SM one CTA of 1024 threads.  Up to a row per SM that is the faster
+// form (64 rows of 4096: 2.1 us, 2.7 with 32 registers); above, a second CTA has to fit: 32 registers.  256 rows of 1024 /
+// 4096 / 16384: 2.8 / 3.8 / 9.2 -> 2.3 / 3.1 / 7.4 us.
+__global__ void __launch_bounds__(1024, 2)
+add_rms_norm_two_kernel(float* __restrict__ x, const float* __restrict__ residual, const float* __restrict__ weight,
+                        int16_t* __restrict__ y, int n, float eps)
+{
+    rms_norm_row<true>(x, residual, weight, y, n, eps);
 }
 
 // SiLU(gate) * up -> bf16 (engine/kernels.hip:447-458), residual add (engine/kernels.hip:340-349)
@@ -1250,7 +1265,7 @@ int launch_add_rms_norm_bf16_batch(float* x, const float* residual, const float*
 {
     if (!x || !residual || !weight || !y || n < 1 || batch_size < 1) return fail(S12_ERR_BAD_ARG, "launch_add_rms_norm_bf16_batch: bad argument");
     const int threads = n >= 1024 ? 1024 : ((n + 31) / 32) * 32;
-    return launch(rms_norm_kernel<true>, dim3(batch_size), dim3(threads), 0, stream, "launch_add_rms_norm_bf16_batch",
+    return launch(threads == 1024 && batch_size > sm_count() ? add_rms_norm_two_kernel : rms_norm_kernel<true>, dim3(batch_size), dim3(threads), 0, stream, "launch_add_rms_norm_bf16_batch",
                   x, residual, weight, y, n, eps);
 }
 int launch_silu_mul_bf16_batch(const float* gate, const float* up, int16_t* out, int n, int batch_size, void* stream)
