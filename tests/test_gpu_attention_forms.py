@@ -41,9 +41,10 @@ def both(n_head, n_kv, hd, lengths, seed=0, edit=None):
 
 def exact(c, b, n, n_head, n_kv, hd):
     g = n_head // n_kv
-    k = c["k"][b, :n].astype(np.float64) * c["sk"][b, :n].astype(np.float64)[..., None]
+    k = c["k"][b, :n].astype(np.float64)
     v = c["v"][b, :n].astype(np.float64) * c["sv"][b, :n].astype(np.float64)[..., None]
     s = np.einsum("hgd,thd->hgt", c["q"][b].astype(np.float64).reshape(n_kv, g, hd), k) / np.sqrt(hd)
+    s *= c["sk"][b, :n].astype(np.float64).T[:, None, :]              # after the sum, as both kernels do
     p = np.exp(s - s.max(axis=-1, keepdims=True))
     p /= p.sum(axis=-1, keepdims=True)
     return np.einsum("hgt,thd->hgd", p, v).reshape(-1), np.einsum("hgt,thd->hgd", p, np.abs(v)).reshape(-1)
@@ -61,10 +62,12 @@ def test_against_float64_and_the_general_kernel(hd, n_head, n_kv, lengths):
         assert (np.abs(new[b] - general[b]) <= 2 * bound).all()
 
 
+@pytest.mark.parametrize("n_head", [8, 16])
 @pytest.mark.parametrize("what", ["q", "sk", "sv", "large"])
-def test_infinities_and_the_largest_values(what):
-    """One infinite input, and value scales near the end of the 32-bit range: the same finite results, infinities and
-    invalid values as the general kernel's."""
+def test_infinities_and_the_largest_values(what, n_head):
+    """One infinite input, and value scales near the end of the 32-bit range.  An invalid 64-bit result is stored as 0x8000
+    (what the rounding to bf16 makes of the hardware's NaN) and an infinity as itself, by both kernels; everything else,
+    such as the heads that the infinity does not touch, is as near to 64 bits as elsewhere."""
     def edit(c):
         if what == "q":
             c["q"][0, 5] = np.inf
@@ -72,12 +75,62 @@ def test_infinities_and_the_largest_values(what):
             c["sv"][0, 3, 0] = 2e36
         else:
             c[what][0, 3, 0] = np.inf
-    _, (new, general) = both(8, 2, 128, (40, 20), seed=3, edit=edit)
-    assert np.array_equal(np.isfinite(new), np.isfinite(general))
-    fine = np.isfinite(new)
-    # bf16 neighbours at most
-    assert (np.abs(new[fine] - general[fine]) <= 2.0 ** -7 * np.abs(general[fine]) + 1e-4).all()
-    assert np.array_equal(np.sign(new[~fine]), np.sign(general[~fine]))
+    lengths, n_kv, hd = (40, 20), 2, 128
+    c, outs = both(n_head, n_kv, hd, lengths, seed=3, edit=edit)
+    with np.errstate(invalid="ignore"):
+        wants = [exact(c, b, n, n_head, n_kv, hd) for b, n in enumerate(lengths)]
+    assert what == "large" or not np.isfinite(wants[0][0]).all()
+    assert np.isfinite(wants[0][0]).any() and np.isfinite(wants[1][0]).all()
+    for out in outs:
+        raw = (out.astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)
+        for b, (want, size) in enumerate(wants):
+            bad, fine = np.isnan(want), np.isfinite(want)
+            assert (raw[b][bad] == 0x8000).all()
+            assert np.array_equal(out[b][~bad & ~fine], want[~bad & ~fine])
+            top = np.repeat(size.reshape(n_head, hd).max(axis=1), hd)[fine]
+            assert (np.abs(out[b][fine] - want[fine]) <= 2.0 ** -8 * np.abs(want[fine]) * (1 + 2.0 ** -8) + 2.0 ** -16 * top).all()
+
+
+def on_device(n_kv, gqa, hd, lengths, seed, off=0):
+    """The call's outputs, and the float64 statement's with the sums of magnitudes, all on the device."""
+    import torch
+    from turbo_lossless_b200 import Split12Engine
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    B, T, n_head = len(lengths), max(lengths), n_kv * gqa
+    kv = [torch.randint(-127, 128, (B * T * n_kv * hd + 16,), dtype=torch.int8, device="cuda", generator=g)[off:] for _ in range(2)]
+    q = torch.randn(B, n_head * hd, device="cuda", generator=g)
+    sk, sv = (0.03 * torch.rand(B, T, n_kv, device="cuda", generator=g) for _ in range(2))
+    pos = torch.tensor(lengths, dtype=torch.int32, device="cuda") - 1
+    out = torch.zeros(B, n_head * hd, dtype=torch.bfloat16, device="cuda")
+    Split12Engine().attention_all_heads_batch(q, kv[0], kv[1], sk, sv, out.view(torch.int16), pos, n_head, n_kv, hd, T, hd ** -0.5, B, T * n_kv * hd)
+    k, v = (t[:B * T * n_kv * hd].view(B, T, n_kv, hd) for t in kv)
+    want, size = [], []
+    for b, n in enumerate(lengths):
+        vb = v[b, :n].double() * sv[b, :n].double()[..., None]
+        s = torch.einsum("hgd,thd->hgt", q[b].double().view(n_kv, gqa, hd), k[b, :n].double() * sk[b, :n].double()[..., None]) * hd ** -0.5
+        p = torch.softmax(s, dim=-1)
+        want.append(torch.einsum("hgt,thd->hgd", p, vb).reshape(-1)); size.append(torch.einsum("hgt,thd->hgd", p, vb.abs()).max())
+    return out.double(), torch.stack(want), torch.stack(size)[:, None]
+
+
+@pytest.mark.parametrize("hd", [64, 96, 128])
+@pytest.mark.parametrize("gqa", [1, 4, 8])
+@pytest.mark.parametrize("lengths", [(2048,), (4099, 2050), (16001,), tuple(range(461, 685)), tuple(range(1500, 1540)) * 3])
+def test_long_enough_to_go_round_the_ring(hd, gqa, lengths):
+    """Warps with four to sixteen chunks, the last one partial, so that every stage of the ring is filled again: few sequences
+    (eight warps a CTA, eight slices), 224 of them (one slice) and 120 (two)."""
+    got, want, size = on_device(2, gqa, hd, lengths, hd + gqa)
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() * (1 + 2.0 ** -8) + 2.0 ** -16 * size).all()
+
+
+@pytest.mark.parametrize("hd,gqa,lengths,off", [(32, 1, (1, 33, 100), 0), (80, 4, (300, 17), 0), (4, 2, (9, 64), 0), (132, 8, (50, 129), 0),
+                                                (256, 1, (200, 1), 0), (256, 2, (77,), 0), (256, 4, (1000, 3), 0), (256, 8, (65, 64), 0),
+                                                (128, 4, (9000,) * 40, 4), (64, 8, (9000, 5000), 4), (256, 4, (9000,) * 40, 0)])
+def test_general_kernel(hd, gqa, lengths, off):
+    """What only the general kernel takes: other head sizes, caches off a 16-byte boundary, and contexts whose slices grow in
+    number until a CTA's scores fit its shared memory (9000 positions)."""
+    got, want, size = on_device(2, gqa, hd, lengths, hd + gqa, off)
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() * (1 + 2.0 ** -8) + 2.0 ** -16 * size).all()
 
 
 @pytest.mark.parametrize("n_kv,gqa,hd,B,T", [(8, 8, 128, 64, 1000), (8, 8, 64, 256, 128), (8, 8, 96, 64, 1000), (8, 4, 128, 56, 7000),

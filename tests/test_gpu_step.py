@@ -194,8 +194,9 @@ def test_batched_rope_store_attention_per_sequence_caches(eng, S):
 def test_flash_attention_names_forward_to_the_same_kernels(eng, S):
     """The engine calls launch_flash_attention[_batch] from position 1024 on (engine/inference.cpp:285,432):
     same arguments, same results as launch_attention_all_heads[_batch], checked against the oracle at 1500
-    positions, and at 9000 positions for 80 (sequence, kv head) pairs with four query heads each: one slice's
-    scores no longer fit a CTA's shared memory, so the positions are cut in two although the GPU is already full."""
+    positions, and at 9000 positions for 80 (sequence, kv head) pairs with four query heads each, with the caches on a
+    16-byte boundary and 4 bytes off it.  The latter takes the general kernel, where one slice's scores do not fit a
+    CTA's shared memory, so that the positions are cut in two although the GPU is already full."""
     import torch
     n_head, n_head_kv, hd, max_seq, seq_len = 32, 8, 128, 2048, 1500
     rng = np.random.default_rng(77)
@@ -228,16 +229,18 @@ def test_flash_attention_names_forward_to_the_same_kernels(eng, S):
     svb = (rng.random((batch, long_seq, n_head_kv)) * 0.02 + 0.001).astype(np.float32)
     pos = rng.integers(7000, long_seq, batch).astype(np.int32)
     pos[0] = long_seq - 1
-    outb = torch.zeros((batch, n_head * hd), dtype=torch.int16, device="cuda")
     dv = [_cuda(a) for a in (qb, kcb, vcb, skb, svb, pos)]          # kept alive until the kernel has run
-    rc = eng.lib.launch_flash_attention_batch(dv[0].data_ptr(), dv[1].data_ptr(), dv[2].data_ptr(), dv[3].data_ptr(),
-                                              dv[4].data_ptr(), outb.data_ptr(), dv[5].data_ptr(), n_head, n_head_kv, hd,
-                                              long_seq, scale, batch, kv_stride, st)
-    assert rc == 0, eng.lib.s12_last_error()
-    torch.cuda.synchronize()
-    for s in (0, 7, batch - 1):
-        want = S.bf16_to_f32(S.attention(qb[s], kcb[s], vcb[s], skb[s], svb[s], int(pos[s]) + 1, n_head, n_head_kv, hd,
-                                         scale)).astype(np.float64)
-        got = S.bf16_to_f32(outb[s].cpu().numpy()).astype(np.float64)
-        assert np.abs(got - want).max() <= 2.0 ** -7 * np.abs(want).max()
+    off_k, off_v = (torch.cat([torch.zeros(4, dtype=torch.int8, device="cuda"), t.flatten()])[4:] for t in dv[1:3])
+    for k_d, v_d in ((dv[1], dv[2]), (off_k, off_v)):
+        outb = torch.zeros((batch, n_head * hd), dtype=torch.int16, device="cuda")
+        rc = eng.lib.launch_flash_attention_batch(dv[0].data_ptr(), k_d.data_ptr(), v_d.data_ptr(), dv[3].data_ptr(),
+                                                  dv[4].data_ptr(), outb.data_ptr(), dv[5].data_ptr(), n_head, n_head_kv, hd,
+                                                  long_seq, scale, batch, kv_stride, st)
+        assert rc == 0, eng.lib.s12_last_error()
+        torch.cuda.synchronize()
+        for s in (0, 7, batch - 1):
+            want = S.bf16_to_f32(S.attention(qb[s], kcb[s], vcb[s], skb[s], svb[s], int(pos[s]) + 1, n_head, n_head_kv, hd,
+                                             scale)).astype(np.float64)
+            got = S.bf16_to_f32(outb[s].cpu().numpy()).astype(np.float64)
+            assert np.abs(got - want).max() <= 2.0 ** -7 * np.abs(want).max()
     assert eng.device_status() == 0
