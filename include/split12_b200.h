@@ -373,7 +373,7 @@ int s12_pack_async(const void* bf16, int M, int K, int base_exp, void* sm, void*
  * them: meta (device, int32 [2]) receives base_exp and the number of escapes,
  * which the caller reads back once; same bytes as the three calls above.
  * scratch: S12_PACK_SCRATCH_BYTES on the device, 8-byte aligned, free again when
- * the call's kernels have run.  M and K at least 1. */
+ * the call's kernels have run.  M at least 1, K even and at least 2. */
 #define S12_PACK_SCRATCH_BYTES (257 * 8)
 int s12_pack_auto_async(const void* bf16, int M, int K, void* scratch, void* meta, void* sm, void* gr,
                         void* row_off, void* stream);

@@ -307,7 +307,7 @@ __device__ __forceinline__ void esc_advance(EscCursor& e, const GemmTensor& T)
 __device__ __forceinline__ void esc_apply(EscCursor& e, const GemmTensor& T, int k0, uint32_t (&v)[32])
 {
     // The columns of the other groups, in a loop of their own: in one loop with the patch, some lane patches in nearly
-    // every round and all wait for it (expert block with 0.25 % escapes 647 -> 606 us).
+    // every round and all wait for it (expert block with 0.25 % escapes, device time, 647 -> 606 us).
     while (e.c0 < k0) esc_advance(e, T);
     while (e.c0 < k0 + kTK) {
         const int idx = e.c0 - k0;
@@ -316,7 +316,7 @@ __device__ __forceinline__ void esc_apply(EscCursor& e, const GemmTensor& T, int
         // quarter (a warp rarely has more than one entry at a time).  Written as PTX so that the register array
         // is not turned into an indexed local-memory array.  With all 32 registers tested for every entry, the
         // escapes cost a tenth of a launch at B = 64 and 0.015 % escapes (28672 x 4096: 47.4 us, 42.0 without them,
-        // 45.9 this way), and a fifth of the time of 14336 x 4096 experts with 0.25 % (whole block 740 -> 653 us).
+        // 45.9 this way), and a tenth of the expert block with 0.25 % (14336 x 4096, issued eagerly, 741 -> 666 us).
         const int h = idx >> 1;
 #pragma unroll
         for (int q = 0; q < 4; q++)

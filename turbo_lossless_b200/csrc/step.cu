@@ -625,7 +625,7 @@ attention_kernel(const __grid_constant__ AttnParams P)
 // warp, sixteen warps per SM (128 registers: q is read from shared memory again for every chunk; with q in registers
 // twelve warps were resident: 31 against 30 us on 256 x 192 positions, 51 against 53 on 24 x 4096).  The partial results
 // of a CTA's warps meet in shared memory, those of a cluster's CTAs over distributed shared memory as above.
-// Measured, 32/8 heads of 128: 24 sequences of 2-4 k positions 195 -> 53 us (3.0 TB/s); bound now by instruction issue
+// Measured, 32/8 heads of 128: 24 sequences of 2-4 k positions 195 -> 54 us (2.9 TB/s); bound now by instruction issue
 // (about 600 instructions a chunk, the ALU pipe half busy with the int8 conversions) and the CTAs' dependent start.
 // ---------------------------------------------------------------------------
 constexpr int kMmaWarps = 8;             // most warps of a CTA
@@ -727,7 +727,7 @@ attention_mma_kernel(const __grid_constant__ AttnParams P)
     auto v_piece = [](int r, int c) { return kHD == 128 ? c ^ (((r >> 1) & 3) << 1) : kHD == 64 ? c ^ (((r >> 1) & 1) << 1) : c; };
     const int first = t_lo + warp * kMmaPos, stride = nwarps * kMmaPos;
     const int n = first < t_hi ? (t_hi - first + stride - 1) / stride : 0;      // this warp's chunks
-    // what a lane copies of a chunk: pieces of rows row0[j], the same in every chunk
+    // what a lane copies of a chunk: pieces j * 32 + lane of its rows, the same in every chunk
     uint32_t src_off[kRowPieces / 2], dst_k[kRowPieces / 2], dst_v[kRowPieces / 2];
 #pragma unroll
     for (int j = 0; j < kRowPieces / 2; j++) {
@@ -919,7 +919,7 @@ attention_mma_kernel(const __grid_constant__ AttnParams P)
     __syncwarp();                                                  // the ring is the warp's own: its partial result goes there
     l += __shfl_xor_sync(0xFFFFFFFFu, l, 1);
     l += __shfl_xor_sync(0xFFFFFFFFu, l, 2);
-    float* mine = reinterpret_cast<float*>(ring);                  // [head][column], padded: see mma_acc_index
+    float* mine = reinterpret_cast<float*>(ring);                  // [head][column], padded: mma_acc_row, mma_acc_col
     const bool owner = kWide || (g < 4 && head < gqa);
 #pragma unroll
     for (int j = 0; j < kTiles; j += 4)
@@ -1131,7 +1131,11 @@ static int rope_kv_launch(RopeKvParams P, bool rope, float theta, int batch, voi
 }
 
 // Launches attention_mma_kernel when it takes the shape (returns its status, 0 or negative), else returns 1.
-// It takes head_dim 64 / 96 / 128 with rows of the caches on 16-byte boundaries.
+// It takes head_dim 64 / 96 / 128 with rows of the caches on 16-byte boundaries, whatever the number of query heads (with
+// one per kv head 3 of the 16 MMA rows are used).  General kernel / this one over 576 sizes (1, 2, 8 kv heads with 1-8 query
+// heads each, 1-256 sequences, 16-16000 positions): at least as fast everywhere, in the middle 1.6x with one query head,
+// 2.0 / 1.8 / 1.7x with heads of 64 / 96 / 128, 1.65x up to 48 positions; nearest at 8 sequences of 100-200 positions with one
+// kv head of 128 (4.9 / 4.9 us).
 static int attention_mma_launch(AttnParams P, int gqa, int max_len, int batch, void* stream, const char* who)
 {
     const int hd = P.head_dim;

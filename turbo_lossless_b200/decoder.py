@@ -72,7 +72,7 @@ class Decoder:
         self.sc_k = torch.zeros(cfg.n_layer, B, cfg.max_seq, cfg.n_head_kv, **f32)
         self.sc_v = torch.zeros_like(self.sc_k)
 
-    # one projection launch: GEMV family for B <= 16, tensor-core GEMM above
+    # one projection launch; a single tensor at 2 <= B <= 16 takes the streaming kernel or, when small, the GEMV family
     def _proj(self, ws, x_bf16, outs):
         if self.B == 1:
             self.eng.gemv(ws, x_bf16, outs)
