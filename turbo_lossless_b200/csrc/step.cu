@@ -626,7 +626,7 @@ attention_kernel(const __grid_constant__ AttnParams P)
 // twelve warps were resident: 31 against 30 us on 256 x 192 positions, 51 against 53 on 24 x 4096).  The partial results
 // of a CTA's warps meet in shared memory, those of a cluster's CTAs over distributed shared memory as above.
 // Measured, 32/8 heads of 128: 24 sequences of 2-4 k positions 195 -> 54 us (2.9 TB/s); bound now by instruction issue
-// (about 600 instructions a chunk, the ALU pipe half busy with the int8 conversions) and the CTAs' dependent start.
+// (about 620 instructions a chunk, the ALU pipe half busy with the int8 conversions) and the CTAs' dependent start.
 // ---------------------------------------------------------------------------
 constexpr int kMmaWarps = 8;             // most warps of a CTA
 constexpr int kMmaPos = 16;              // positions of a chunk
@@ -1143,7 +1143,8 @@ static int attention_mma_launch(AttnParams P, int gqa, int max_len, int batch, v
         ((reinterpret_cast<uintptr_t>(P.kc) | reinterpret_cast<uintptr_t>(P.vc)) & 15) != 0)
         return 1;
     // Slices while three CTAs per SM (four are resident) are not there, of 64 positions or more: a CTA costs ~6 us of
-    // dependent loads and merging whatever its length.  32/8 heads of 128, us with 1 / 2 / 4 / 8 slices: 24 sequences of
+    // dependent loads and merging whatever its length.  32/8 heads of 128, us with 1 / 2 / 4 / 8 slices (as first built,
+    // with chained accumulators; within 4 % of now): 24 sequences of
     // 4096 77 / 67 / 53 / 53; 64 of 1000 36 / 37 / 42 / 60; 256 of 192 30 / 53 / 84 / 168; one of 8000 100 / 54 / 29 / 17.
     int nsplit = 1;
     const long long pairs = (long long)P.n_head_kv * batch;
