@@ -188,3 +188,20 @@ def test_positions_past_the_bound_read_nothing_past_it(hd, off, bound):
         eng.attention_all_heads_batch(q, kv[0][off:], kv[1][off:], sk, sv, out, pos, 8, n_kv, hd, bound, hd ** -0.5, B, room * n_kv * hd)
         outs.append(out)
     assert outs[0].any() and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("hd,gqa", [(64, 1), (96, 8), (128, 4), (128, 8)])
+@pytest.mark.parametrize("length", [20, 130, 600])
+def test_output_off_an_eight_byte_boundary(hd, gqa, length):
+    """The same bits wherever the output starts: one slice and several, merged one and four elements a thread."""
+    import torch
+    from turbo_lossless_b200 import Split12Engine
+    g = torch.Generator(device="cuda").manual_seed(length)
+    k, v = (torch.randint(-127, 128, (length * hd,), dtype=torch.int8, device="cuda", generator=g) for _ in range(2))
+    q, sk, sv = torch.randn(gqa * hd, device="cuda", generator=g), *(0.03 * torch.rand(length, device="cuda", generator=g) for _ in range(2))
+    room = torch.zeros(3, gqa * hd + 4, dtype=torch.int16, device="cuda")
+    pos = torch.full((1,), length - 1, dtype=torch.int32, device="cuda")
+    for i in range(3):                                             # rows of a multiple of 8 bytes: 0, 2 and 4 bytes off
+        Split12Engine().attention_all_heads_batch(q, k, v, sk, sv, room[i, i:], pos, gqa, 1, hd, length, hd ** -0.5, 1, length * hd)
+    assert room[0].any() and all(torch.equal(room[0, :gqa * hd], room[i, i:i + gqa * hd]) for i in (1, 2))
+    assert not room[1, 0] and not room[0, gqa * hd:].any()
