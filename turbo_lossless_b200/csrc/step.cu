@@ -71,8 +71,9 @@ embed_kernel(const int16_t* __restrict__ table, const int* __restrict__ tokens, 
 // (engine/kernels.hip:355-393, 399-442).  One CTA per sequence.
 // ---------------------------------------------------------------------------
 // Bound by latency: rows that fit the CTA's registers (two 16-byte pieces a thread) are read once, together with their
-// weights.  Rows of 4096 with the residual, in a chain of launches: 2.6 -> 1.9 us at B = 1, 3.8 us at B = 256 as before.
-template <bool kAdd>
+// weights.  Rows of 4096 with the residual, in a chain of launches: 2.6 -> 1.9 us at B = 1, 3.7 -> 3.1 us at B = 256.  kLong:
+// the row is longer than that; without the other branch beside it, 64 rows of 16384 take 4.5 us instead of 4.7.
+template <bool kAdd, bool kLong = false>
 __device__ __forceinline__ void rms_norm_row(float* __restrict__ x, const float* __restrict__ residual, const float* __restrict__ weight,
                                              int16_t* __restrict__ y, int n, float eps)
 {
@@ -92,7 +93,7 @@ __device__ __forceinline__ void rms_norm_row(float* __restrict__ x, const float*
     };
     float ss = 0.f;
     grid_dependency_wait();
-    if (vec && n / 4 <= 2 * (int)blockDim.x) {
+    if (!kLong && vec && n / 4 <= 2 * (int)blockDim.x) {
         float4 v[2], w[2], r[2];
 #pragma unroll
         for (int j = 0; j < 2; j++) {
@@ -135,12 +136,12 @@ __device__ __forceinline__ void rms_norm_row(float* __restrict__ x, const float*
     for (int i = threadIdx.x; i < n; i += blockDim.x)
         y[off + i] = float_to_bf16_rne(x[off + i] * rms * weight[i]);    // a thread re-reads only what it wrote
 }
-template <bool kAdd>
+template <bool kAdd, bool kLong = false>
 __global__ void __launch_bounds__(1024)
 rms_norm_kernel(float* __restrict__ x, const float* __restrict__ residual, const float* __restrict__ weight,
                 int16_t* __restrict__ y, int n, float eps)
 {
-    rms_norm_row<kAdd>(x, residual, weight, y, n, eps);
+    rms_norm_row<kAdd, kLong>(x, residual, weight, y, n, eps);
 }
 // With the residual a thread takes 48 registers, and an SM one CTA of 1024 threads.  Up to a row per SM that is the faster
 // form (64 rows of 4096: 2.1 us, 2.7 with 32 registers); above, a second CTA has to fit: 32 registers.  256 rows of 1024 /
@@ -1262,7 +1263,7 @@ int launch_rms_norm_bf16_batch(const float* x, const float* weight, int16_t* y, 
 {
     if (!x || !weight || !y || n < 1 || batch_size < 1) return fail(S12_ERR_BAD_ARG, "launch_rms_norm_bf16_batch: bad argument");
     const int threads = n >= 1024 ? 1024 : ((n + 31) / 32) * 32;
-    return launch(rms_norm_kernel<false>, dim3(batch_size), dim3(threads), 0, stream, "launch_rms_norm_bf16_batch",
+    return launch(n > 8192 ? rms_norm_kernel<false, true> : rms_norm_kernel<false>, dim3(batch_size), dim3(threads), 0, stream, "launch_rms_norm_bf16_batch",
                   const_cast<float*>(x), (const float*)nullptr, weight, y, n, eps);
 }
 int launch_add_rms_norm_bf16_batch(float* x, const float* residual, const float* weight, int16_t* y, int n, float eps,
